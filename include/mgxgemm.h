@@ -107,7 +107,7 @@ MGX_API int mgx_validate_matrix_c(const double *d_c, int rows, int cols, double 
 MGX_API int mgx_gemm_fp64(const double *A, const double *B, double *C, int m, int n, int k, int lda, int ldb,
                           int ldc, int beta_one, void *stream);
 
-/* Split-K form for products with too few 128 x 128 output tiles to fill the GPU: the K range is
+/* Split-K form for products whose output is too small to fill the GPU: the K range is
  * cut into `ksplit` slices (at most one per 32-wide K block) computed by separate CTAs, and the
  * slice products are summed into C in slice order (deterministic).  The rounding differs from
  * mgx_gemm_fp64 by the slice sums.  No counterpart in MGXBench; the autotuner picks ksplit.
@@ -118,17 +118,17 @@ MGX_API int mgx_gemm_fp64_splitk(const double *A, const double *B, double *C, in
                                  int ldb, int ldc, int beta_one, int ksplit, void *workspace,
                                  size_t workspace_bytes, void *stream);
 
-/* mgx_gemm_fp64_splitk with a choice of output tile: tile_m = 128 (128 x 128 tiles, the default
- * of every other FP64 entry point) or 64 (64 x 128 tiles: twice the work items, for products with
- * few 128 x 128 tiles on the 148 SMs).  No counterpart in MGXBench; the autotuner's tile
- * candidates pick it.  Both tiles reduce every element over K in the same order, so the result
- * does not depend on tile_m.  ksplit and workspace as for mgx_gemm_fp64_splitk. */
+/* mgx_gemm_fp64_splitk with a choice of output tile, tile_m = 64 or 128, of the autotuner's tile
+ * candidates (no counterpart in MGXBench).  Every element is reduced over K in the same order
+ * whatever the tile, so the result does not depend on tile_m; the kernel now cuts every product
+ * into equal shares of 64-row bands, so the speed does not either.  ksplit and workspace as for
+ * mgx_gemm_fp64_splitk. */
 MGX_API int mgx_gemm_fp64_tiled(const double *A, const double *B, double *C, int m, int n, int k, int lda, int ldb,
                                 int ldc, int beta_one, int tile_m, int ksplit, void *workspace,
                                 size_t workspace_bytes, void *stream);
 
-/* Stream-K form of the FP64 product over 64 x 128 tiles, for products with too few tiles to fill
- * the GPU (no counterpart in MGXBench; the autotuner offers it).  Every CTA takes an equal
+/* Stream-K form of the FP64 product over 64-row tiles of up to 128 columns, for products whose
+ * output is too small to fill the GPU (no counterpart in MGXBench; the autotuner offers it).  Every CTA takes an equal
  * share of all tiles' 32-wide K blocks, so every SM has the same work; a tile whose K range is
  * split between CTAs is finished by the last of them to arrive, which adds the pieces in K order.
  * No CTA waits for another.  Deterministic for a given GPU (the shares depend on its SM count),
@@ -290,20 +290,20 @@ typedef struct {
 
 typedef struct mgx_summa_plan mgx_summa_plan_t;
 
-/* The FP64 plan's work list, computed on the host: returns the number of work tiles and writes up
- * to `capacity` of them to out as {m0, n_lo, m_end, n_end} (columns [n_lo, n_end) of rows
- * [m0, m_end)).  Needs no device. */
+/* The blocks of an FP64 plan as 128 x 128 work tiles, computed on the host: returns the number of
+ * tiles and writes up to `capacity` of them to out as {m0, n_lo, m_end, n_end} (columns
+ * [n_lo, n_end) of rows [m0, m_end)).  Needs no device. */
 MGX_API int mgx_summa_tiles(const mgx_summa_desc_t *desc, int *out, int capacity);
 
-/* Builds the work list on the current device and allocates the Ozaki workspace if needed. */
+/* Checks the grid and allocates the Ozaki workspace if needed, on the current device. */
 MGX_API int mgx_summa_plan_create(const mgx_summa_desc_t *desc, mgx_summa_plan_t **plan);
 
 /* C = SUMMA product of A (m x k, lda) and B (k x n, ldb); stream-ordered, allocates nothing. */
 MGX_API int mgx_summa_run(mgx_summa_plan_t *plan, const double *A, int lda, const double *B, int ldb, double *C,
                           int ldc, void *stream);
 
-/* Work tiles, K steps and workspace bytes of a plan.  FP64 form: the persistent kernel's 128 x 128
- * tiles clipped to their blocks, and the panels it accumulates in order.  The Ozaki and CRT forms
+/* Work tiles, K steps and workspace bytes of a plan.  FP64 form: the 128 x 128 tiles of
+ * mgx_summa_tiles, and the panels the persistent kernel accumulates in order.  The Ozaki and CRT forms
  * use no panel list: their integer sums are exact and their scales belong to whole rows and
  * columns, so neither the block cuts nor the panel order change a bit of C, and the plan runs one
  * product of all of C.  For them work_tiles is that product's work items (128 x 128 tiles for the

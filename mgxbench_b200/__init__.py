@@ -190,9 +190,9 @@ def fp64_splitk_workspace_size(m, n, k, ksplit) -> int:
 
 def gemm_fp64(A, B, C, beta_one: bool = False, stream=None, ksplit: int = 1, workspace=None, tile_m: int = 128):
     """C (+)= A B on the FP64 tensor cores; ksplit > 1 cuts K into slices computed by separate
-    CTAs (for products with few output tiles) and needs a workspace (grown on demand); tile_m = 64
-    runs 64 x 128 output tiles instead of 128 x 128 (same result, bit for bit); ksplit = 0 is the
-    stream-K form over 64 x 128 tiles (equal K shares per CTA, workspace grown on demand)."""
+    CTAs (for products with few output tiles) and needs a workspace (grown on demand); tile_m (64
+    or 128) changes neither the result nor the speed; ksplit = 0 is the stream-K form (equal K shares
+    per CTA, workspace grown on demand)."""
     _check_f64(A, B, C)
     m, k = A.shape
     n = B.shape[1]

@@ -243,10 +243,10 @@ int mgx_launch_dgemm_streamk(const double *A, const double *B, double *C, int m,
                              int ldc, int beta_one, void *workspace, size_t workspace_bytes, cudaStream_t stream);
 int mgx_launch_dgemm_splitk(const double *A, const double *B, double *C, int m, int n, int k, int lda, int ldb,
                             int ldc, int beta_one, int ksplit, void *partial, size_t partial_bytes,
-                            cudaStream_t stream, int tile_m = 128);
+                            cudaStream_t stream);
 
 int mgx_launch_dgemm(const double *A, const double *B, double *C, int m, int n, int k_len, int a_x0, int a_x_end,
-                     int b_rows, int lda, int ldb, int ldc, int beta_one, cudaStream_t stream, int force_generic);
+                     int b_rows, int lda, int ldb, int ldc, int beta_one, cudaStream_t stream);
 int mgx_validate_impl(const double *d_c, size_t count, double expected, double abs_tol, double rel_tol,
                       mgx_validation_t *out, cudaStream_t stream);
 
@@ -336,7 +336,7 @@ MGX_API int mgx_gemm_fp64(const double *A, const double *B, double *C, int m, in
                              ldb, ldc);
         return MGX_E_INVALID;
     }
-    return mgx_launch_dgemm(A, B, C, m, n, k, 0, k, k, lda, ldb, ldc, beta_one ? 1 : 0, (cudaStream_t)stream, 0);
+    return mgx_launch_dgemm(A, B, C, m, n, k, 0, k, k, lda, ldb, ldc, beta_one ? 1 : 0, (cudaStream_t)stream);
 }
 
 MGX_API size_t mgx_fp64_splitk_workspace_size(int m, int n, int k, int ksplit)
@@ -373,7 +373,7 @@ MGX_API int mgx_gemm_fp64_streamk(const double *A, const double *B, double *C, i
         return MGX_E_INVALID;
     }
     if (m == 0 || n == 0 || k == 0)
-        return mgx_launch_dgemm(A, B, C, m, n, k, 0, k, k, lda, ldb, ldc, beta_one ? 1 : 0, (cudaStream_t)stream, 0);
+        return mgx_launch_dgemm(A, B, C, m, n, k, 0, k, k, lda, ldb, ldc, beta_one ? 1 : 0, (cudaStream_t)stream);
     return mgx_launch_dgemm_streamk(A, B, C, m, n, k, lda, ldb, ldc, beta_one ? 1 : 0, workspace, workspace_bytes,
                                     (cudaStream_t)stream);
 }
@@ -390,7 +390,7 @@ MGX_API int mgx_gemm_fp64_tiled(const double *A, const double *B, double *C, int
         return MGX_E_INVALID;
     }
     return mgx_launch_dgemm_splitk(A, B, C, m, n, k, lda, ldb, ldc, beta_one ? 1 : 0, ksplit, workspace,
-                                   workspace_bytes, (cudaStream_t)stream, tile_m);
+                                   workspace_bytes, (cudaStream_t)stream);
 }
 
 MGX_API int mgx_ab_multiply(double *a, double *b, double *c, int m, int n, int k, int lda, int ldb, int ldc, int w)
@@ -414,14 +414,11 @@ MGX_API int mgx_ab_multiply_accumulate_async(const double *a, const double *b_ch
     if (m == 0 || n == 0 || k_chunk == 0) return MGX_SUCCESS;
     int a_x_end = k_offset + k_chunk;
     if (a_x_end > k_total) a_x_end = k_total;
-    if (a_x_end <= k_offset) {
-        // Every A column of the chunk is outside k_total: the reference multiplies zeros.
-        // Route it through the generic kernel so 0 * B keeps the reference's NaN behaviour.
-        return mgx_launch_dgemm(a, b_chunk, c, m, n, k_chunk, k_offset, k_offset, k_chunk, lda, ldb, ldc, 1,
-                                (cudaStream_t)stream, 1);
-    }
+    // Where every A column of the chunk is outside k_total the reference multiplies zeros, which
+    // keeps 0 * B's NaN behaviour: A then reads as zero and B as it is.
+    if (a_x_end < k_offset) a_x_end = k_offset;
     return mgx_launch_dgemm(a, b_chunk, c, m, n, k_chunk, k_offset, a_x_end, k_chunk, lda, ldb, ldc, 1,
-                            (cudaStream_t)stream, 0);
+                            (cudaStream_t)stream);
 }
 
 MGX_API int mgx_validate_matrix_c(const double *d_c, int rows, int cols, double expected, double abs_tol,

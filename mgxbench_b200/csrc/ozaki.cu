@@ -1042,7 +1042,7 @@ extern "C" MGX_API int mgx_ozaki_kmax(int splits)
 // one mgx_gemm_ozaki / mgx_gemm_fp64 call (exponents per row of A and per column of B over the
 // whole K), so the result is bit-identical to it.
 int mgx_launch_dgemm(const double *A, const double *B, double *C, int m, int n, int k_len, int a_x0, int a_x_end,
-                     int b_rows, int lda, int ldb, int ldc, int beta_one, cudaStream_t stream, int force_generic);
+                     int b_rows, int lda, int ldb, int ldc, int beta_one, cudaStream_t stream);
 
 // CRT form hooks (ozaki_crt.cu): whole-product workspace, panel preparation, block products.
 size_t mgx_crt_host_ws_bytes(int M, int N, int K, int q);
@@ -1176,8 +1176,7 @@ extern "C" MGX_API int mgx_gemm_host(const double *hA, const double *hB, double 
         } else if (crt) {
             rc = mgx_crt_host_block(Cb, n, r0, c0, r1 - r0, c1 - c0, m, n, k, splits, ws, cs, blk & 1);
         } else {
-            rc = mgx_launch_dgemm(dA + (size_t)r0 * kk, dB + c0, Cb, r1 - r0, c1 - c0, k, 0, k, k, (int)kk, n, n, 0, cs,
-                                  0);
+            rc = mgx_launch_dgemm(dA + (size_t)r0 * kk, dB + c0, Cb, r1 - r0, c1 - c0, k, 0, k, k, (int)kk, n, n, 0, cs);
         }
         fail(cudaEventRecord(evBlk[blk], cs), "record");
         fail(cudaStreamWaitEvent(sout, evBlk[blk], 0), "wait");

@@ -3,21 +3,22 @@
 // The reference runs one process per block (2D-block-matrix/mmb.cu:94-109) and, for every panel
 // k0 of width BK, broadcasts A_i[:, k0:k0+kc] along its process row and B_j[k0:k0+kc, :] along
 // its process column before C_ij += A_panel B_panel (mmb.cu:239-361).  Here A and B are resident,
-// so a plan turns the grid into a list of 128 x 128 work tiles clipped to their blocks, and one
-// persistent kernel walks (tile, panel) in order: the FP64 form adds each panel's product into
-// C_ij with one rounding, as the reference does.  The Ozaki form accumulates the panels exactly
-// in int32 and recombines once; because its element values do not depend on how the output is
-// tiled, it covers every block with one uniform 128 x 128 raster of the whole C.  The CRT form
-// likewise: its scales belong to whole rows of A and columns of B and its residue sums are exact,
-// so all blocks run as one CRT product of the whole C.
+// and one persistent kernel computes every block and panel: the FP64 form adds each panel's product
+// into the element's running sum with one rounding, as the reference does.  An element's value
+// depends on the panel boundaries but not on the block it falls in, so all forms cover C with
+// one uniform raster, whatever the block cuts: the FP64 kernel in equal shares of 64-row bands, the
+// Ozaki form in 128 x 128 tiles (panels accumulate exactly in int32 and are recombined once), the
+// CRT form as one product (its scales belong to whole rows of A and columns of B and its residue
+// sums are exact).
 #include <cstring>
 #include <vector>
 
 #include "mgx_common.cuh"
 
-int mgx_launch_dgemm_ex(const double *A, const double *B, double *C, int m, int n, int k_len, int a_x0, int a_x_end,
-                        int b_rows, int lda, int ldb, int ldc, int beta_one, cudaStream_t stream, int force_generic,
-                        const int4 *tiles, int num_tiles, int panel_kb);
+int mgx_launch_dgemm(const double *A, const double *B, double *C, int m, int n, int k_len, int a_x0, int a_x_end,
+                     int b_rows, int lda, int ldb, int ldc, int beta_one, cudaStream_t stream);
+int mgx_launch_dgemm_panels(const double *A, const double *B, double *C, int m, int n, int k, int lda, int ldb,
+                            int ldc, int panel_k, cudaStream_t stream);
 int mgx_ozaki_run(const double *A, const double *B, double *C, int m, int n, int k, int lda, int ldb, int ldc,
                   int beta_one, int splits, void *workspace, size_t workspace_bytes, cudaStream_t stream);
 int mgx_crt_run(const double *A, const double *B, double *C, int m, int n, int k, int lda, int ldb, int ldc,
@@ -26,7 +27,6 @@ int mgx_crt_run(const double *A, const double *B, double *C, int m, int n, int k
 struct mgx_summa_plan {
     mgx_summa_desc_t desc;
     std::vector<int> rcut, ccut;
-    int4 *d_tiles = nullptr;
     int num_tiles = 0;
     void *ws = nullptr;
     size_t ws_bytes = 0;
@@ -49,10 +49,9 @@ static bool cuts_ok(const std::vector<int> &c, int extent)
     return true;
 }
 
-// Work tiles, block by block in rank order: {m0, n_lo, m_end, n_end}.  Rows start at the block's
-// first row.  Column tiles start at the block's first column rounded down to even (the kernel's
-// B boxes need an even column); n_lo keeps the block's exact first column so the kernel never
-// stores into the neighbouring block.
+// Work tiles of the FP64 form, block by block in rank order: {m0, n_lo, m_end, n_end}.  Rows start
+// at the block's first row.  Column tiles start at the block's first column rounded down to even (a
+// TMA box of B needs an even column); n_lo is the block's exact first column.
 static std::vector<int4> summa_tiles(const std::vector<int> &rcut, const std::vector<int> &ccut)
 {
     std::vector<int4> tiles;
@@ -118,14 +117,11 @@ MGX_API int mgx_summa_plan_create(const mgx_summa_desc_t *desc, mgx_summa_plan_t
         mgx_set_last_message("mgx_summa_plan_create: block cuts must rise strictly from 0 to the extent");
         return MGX_E_INVALID;
     }
-    std::vector<int4> tiles = summa_tiles(P->rcut, P->ccut);
-    P->num_tiles = (int)tiles.size();
-    cudaGetDevice(&P->device);
-    if (cudaMalloc(&P->d_tiles, tiles.size() * sizeof(int4)) != cudaSuccess ||
-        cudaMemcpy(P->d_tiles, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice) != cudaSuccess) {
-        mgx_set_last_message("mgx_summa_plan_create: could not store the work list on the device");
-        if (P->d_tiles) cudaFree(P->d_tiles);
+    P->num_tiles = (int)summa_tiles(P->rcut, P->ccut).size();
+    if (cudaGetDevice(&P->device) != cudaSuccess) {
+        cudaGetLastError();
         delete P;
+        mgx_set_last_message("mgx_summa_plan_create: no CUDA device");
         return MGX_E_CUDA;
     }
     if (desc->form == MGX_FORM_OZAKI || desc->form == MGX_FORM_CRT) {
@@ -133,7 +129,6 @@ MGX_API int mgx_summa_plan_create(const mgx_summa_desc_t *desc, mgx_summa_plan_t
                                                    : mgx_crt_workspace_size(desc->m, desc->n, desc->k, desc->splits);
         if (cudaMalloc(&P->ws, P->ws_bytes) != cudaSuccess) {
             mgx_set_last_message("mgx_summa_plan_create: workspace of %zu bytes", P->ws_bytes);
-            cudaFree(P->d_tiles);
             delete P;
             return MGX_E_CUDA;
         }
@@ -155,17 +150,15 @@ MGX_API int mgx_summa_run(mgx_summa_plan_t *P, const double *A, int lda, const d
         return mgx_ozaki_run(A, B, C, d.m, d.n, d.k, lda, ldb, ldc, 0, d.splits, P->ws, P->ws_bytes, s);
     if (d.form == MGX_FORM_CRT)  // likewise: one CRT product of the whole C
         return mgx_crt_run(A, B, C, d.m, d.n, d.k, lda, ldb, ldc, 0, d.splits, P->ws, P->ws_bytes, s);
-    // C = 0 (2D-block-matrix/mmb.cu:186), then every panel adds into it.
-    MGX_HOST_CHECK(cudaMemset2DAsync(C, (size_t)ldc * sizeof(double), 0, (size_t)d.n * sizeof(double), d.m, s));
-    const int bk = d.panel_k < d.k ? d.panel_k : d.k;
-    if (bk % 32 == 0)
-        return mgx_launch_dgemm_ex(A, B, C, d.m, d.n, d.k, 0, d.k, d.k, lda, ldb, ldc, 1, s, 0, P->d_tiles,
-                                   P->num_tiles, bk / 32);
-    // Panels that do not align with the kernel's 32-wide K blocks: one launch per panel.
-    for (int k0 = 0; k0 < d.k; k0 += bk) {
-        const int kc = (d.k - k0 < bk) ? d.k - k0 : bk;
-        const int rc = mgx_launch_dgemm_ex(A, B + (size_t)k0 * ldb, C, d.m, d.n, kc, k0, k0 + kc, kc, lda, ldb, ldc, 1,
-                                           s, 0, P->d_tiles, P->num_tiles, 0);
+    // C = 0 (2D-block-matrix/mmb.cu:186), then every panel adds into it, in one kernel
+    if (d.panel_k % 32 == 0 || d.panel_k >= d.k)
+        return mgx_launch_dgemm_panels(A, B, C, d.m, d.n, d.k, lda, ldb, ldc, d.panel_k, s);
+    // Panels that do not align with the kernel's 32-wide K blocks: one launch per panel, the first
+    // of which writes C (0 + its product).
+    for (int k0 = 0; k0 < d.k; k0 += d.panel_k) {
+        const int kc = (d.k - k0 < d.panel_k) ? d.k - k0 : d.panel_k;
+        const int rc = mgx_launch_dgemm(A, B + (size_t)k0 * ldb, C, d.m, d.n, kc, k0, k0 + kc, kc, lda, ldb, ldc, k0 > 0,
+                                        s);
         if (rc != MGX_SUCCESS) return rc;
     }
     return MGX_SUCCESS;
@@ -196,7 +189,6 @@ MGX_API int mgx_summa_plan_info(const mgx_summa_plan_t *P, int *work_tiles, int 
 MGX_API int mgx_summa_plan_destroy(mgx_summa_plan_t *P)
 {
     if (!P) return MGX_SUCCESS;
-    if (P->d_tiles) cudaFree(P->d_tiles);
     if (P->ws) cudaFree(P->ws);
     delete P;
     return MGX_SUCCESS;
