@@ -135,17 +135,23 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
 }
 
 // Bounded wait for waits expected to be long (a warp idling through a whole phase of another
-// role's work): polls with a growing nanosleep so the waiting warp leaves the issue slots to
-// the warps doing the work.
+// role's work): each try suspends the warp in hardware for up to kSuspendNs, so it leaves the issue
+// slots to the warps doing the work and still resumes as soon as the phase completes.
+constexpr uint32_t kSuspendNs = 4000;
+
 __device__ __forceinline__ bool mbar_wait_sleepy(uint64_t *bar, uint32_t parity, int *status, int code)
 {
-    if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
-    unsigned ns = 64;
     while (true) {
-        __nanosleep(ns);
-        if (mbar_try_wait(bar, parity)) return true;
-        if (ns < 2048) ns <<= 1;
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendNs)
+            : "memory");
+        if (ok) return true;
         if (global_ns() - t0 > kWaitLimitNs) {
             record_status(status, code);
             return false;
