@@ -37,6 +37,7 @@
 //                   each): tcgen05.ld, exact reduction mod p_l (biased Barrett), one byte per output
 //   crt_combine     CRT recombination of the q residue planes, scaling, (C +) store
 // All waits are bounded (mgx_common.cuh); TMEM is always released before the CTA exits.
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 
@@ -83,10 +84,12 @@ static const int h_moduli[MAXQ] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 
 
 // Host-computed constants of one modulus set.
 struct Consts {
-    int q, L, alpha, beta, E3;
-    double w[MAXQ][3];     // CRT weights in 40-bit chunks
-    double pc[3];          // P in 40-bit chunks
-    double inv_phat;       // 1 / (P / 2^(L-40))
+    int q, L, alpha, beta;
+    int E3;                // L - 120 + 60
+    // CRT recombination, scaled by powers of two (see crt_combine)
+    double w[MAXQ][3];     // CRT weights in 40-bit chunks, 2^974
+    double pc[3];          // P in 40-bit chunks, 2^-60
+    double inv_phat;       // 2^60 / (P / 2^(L-40))
     double c32[MAXQ];      // 2^32 mod p_l
     double inv_p[MAXQ];    // 1 / p_l (rounded)
     uint32_t barrett[MAXQ];  // ceil(2^32 / p_l)
@@ -707,7 +710,22 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
 // Product residues of one 256 x 256 tile are stored [h][quarter][8-column chunk][lane][8 B]: the
 // epilogue warp of TMEM lane quarter `quarter` and accumulator h writes 256 contiguous bytes per
 // chunk.  One warp here takes one (tile, h, quarter, chunk): lane = row within the quarter,
-// 8 columns.  beta_one: C (+)= result.
+// 8 columns.  Where C's rows are 32-byte aligned a lane stores its own 64 bytes, two whole sectors.
+// Elsewhere these would be partial sectors, so the block's 8 warps, which hold 64 consecutive columns
+// of the same 32 rows, pass through shared memory and write 512-byte row pieces (2501 x 1999: 41 us
+// by 8-byte stores, 33 staged; 2496 x 2000: 33 staged, 29 by 32-byte stores).
+// beta_one: C (+)= result.
+//
+// Bound by the FP64 pipe, three multiply-adds per residue.  A residue byte R becomes an FP64 operand
+// by one byte permute: as byte 1 of the high word it is the subnormal R 2^-1034, and the weights
+// carry 2^974, so the sums come out as s 2^-60, exact as before (no bit is lost: they are multiples
+// of 2^-60 below 2^-8).  P's chunks and the exponents carry the same 2^60, which no rounding sees.
+// Before, an add turned 2^52 + R into R, every scale factor was built and range-checked per element,
+// and rint was a conversion: 152 instructions per output, 39-41 us there and 424 us at 8192 x 8192 (347
+// now: 1.54 GB of residues and C, 4.4 TB/s).
+constexpr int kCombineShift = 60;
+constexpr int COMBINE_LD = 66;  // doubles of a staged row: 16-byte stores of 8 lanes hit every bank once
+
 struct CombineParams {
     const uint8_t *rc;        // the block's first tile of the residue planes
     size_t rc_mod;
@@ -722,77 +740,137 @@ struct CombineParams {
 // SPLITK: the residue planes of p.ksplit K slices are added modulo p first (a separate
 // instantiation with a larger register budget, so the whole-K kernel keeps its own).
 template <int Q, bool SPLITK>
-__global__ void __launch_bounds__(256, SPLITK ? 2 : 3) crt_combine(const __grid_constant__ CombineParams p, long long units)
+__global__ void __launch_bounds__(256, SPLITK ? 2 : 3) crt_combine(const __grid_constant__ CombineParams p)
 {
     const int lane = threadIdx.x & 31;
-    const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (unit >= units) return;
+    __shared__ __align__(16) double out[32][COMBINE_LD];
+    const int warp = threadIdx.x >> 5;
+    const long long unit = (long long)blockIdx.x * 8 + warp;
     const int c = (int)(unit & 31), qd = (int)((unit >> 5) & 3), h = (int)((unit >> 7) & 1);
     const long long tile = unit >> 8;
     const int tm = (int)(tile / p.tiles_n), tn = (int)(tile % p.tiles_n);
-    const int row = tm * TILE + h * 128 + qd * 32 + lane;
+    const int row0 = tm * TILE + h * 128 + qd * 32, row = row0 + lane;
     const int col0 = tn * TILE + c * 8;
-    if (row >= p.m || col0 >= p.n) return;
+    if (row0 >= p.m || tn * TILE + (c & ~7) * 8 >= p.n) return;  // the whole block is outside
     const uint8_t *src = p.rc + ((size_t)tm * p.rc_tile_ld + tn) * OUT_TILE_BYTES +
                          (size_t)((h * 4 + qd) * 32 + c) * 256 + lane * 8;
-    double s1[8], s2[8], s3[8];
+    uint2 res[Q];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) s1[j] = s2[j] = s3[j] = 0.0;
+    for (int l = 0; l < Q; ++l) res[l] = __ldg(reinterpret_cast<const uint2 *>(src + (size_t)l * p.rc_mod));
+    const int srow = row < p.m ? p.sg[row] : 0;
+    int e[8];  // the outputs' exponents
+    bool plain = srow != NONFINITE;
 #pragma unroll
-    for (int l = 0; l < Q; ++l) {
-        uint32_t res[8];
-        const uint2 v = __ldg(reinterpret_cast<const uint2 *>(src + (size_t)l * p.rc_mod));
+    for (int j = 0; j < 8; ++j) {
+        const int scol = p.tu[min(col0 + j, p.n - 1)];
+        plain = plain && scol != NONFINITE;
+        e[j] = p.K.E3 - srow - scol;
+    }
+    if (SPLITK) {
+        // the slices' residues (each < p) add modulo p
 #pragma unroll
-        for (int j = 0; j < 8; ++j) res[j] = ((j < 4 ? v.x : v.y) >> (8 * (j & 3))) & 255u;
-        if (SPLITK) {
-            // the slices' residues (each < p) add modulo p
+        for (int l = 0; l < Q; ++l) {
+            uint32_t r[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) r[j] = ((j < 4 ? res[l].x : res[l].y) >> (8 * (j & 3))) & 255u;
             for (int t = 1; t < p.ksplit; ++t) {
                 const uint2 u = __ldg(reinterpret_cast<const uint2 *>(src + (size_t)t * p.rc_slice + (size_t)l * p.rc_mod));
 #pragma unroll
-                for (int j = 0; j < 8; ++j) res[j] += ((j < 4 ? u.x : u.y) >> (8 * (j & 3))) & 255u;
+                for (int j = 0; j < 8; ++j) r[j] += ((j < 4 ? u.x : u.y) >> (8 * (j & 3))) & 255u;
             }
 #pragma unroll
-            for (int j = 0; j < 8; ++j) res[j] = mod_p((int32_t)res[j], (uint32_t)c_moduli[l], p.K.barrett[l]);
-        }
-        const double w1 = p.K.w[l][0], w2 = p.K.w[l][1], w3 = p.K.w[l][2];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            // (double) of a residue: 2^52 + r from the bit pattern, minus 2^52 (exact)
-            const double r = __dsub_rn(__hiloint2double(0x43300000, res[j]), 4503599627370496.0);
-            s1[j] = __fma_rn(w1, r, s1[j]);
-            s2[j] = __fma_rn(w2, r, s2[j]);
-            s3[j] = __fma_rn(w3, r, s3[j]);
+            for (int j = 0; j < 8; ++j) r[j] = mod_p((int32_t)r[j], (uint32_t)c_moduli[l], p.K.barrett[l]);
+            res[l] = make_uint2(r[0] | r[1] << 8 | r[2] << 16 | r[3] << 24, r[4] | r[5] << 8 | r[6] << 16 | r[7] << 24);
         }
     }
-    const int srow = p.sg[row];
-    double *crow = p.C + (size_t)row * p.ldc;
+    // plain: every scale is finite and every exponent within one normal factor (as a rule)
 #pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-        double v[2];
+    for (int j = 0; j < 8; ++j) plain = plain && e[j] >= -1022 && e[j] <= 1023;
+    plain = __all_sync(0xffffffffu, plain);
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int col = col0 + j + u;
-            const int scol = col < p.n ? p.tu[col] : 0;
-            const double Qd = rint(__dmul_rn(__fma_rn(s2[j + u], 0x1p-40, s1[j + u]), p.K.inv_phat));
-            const double d1 = __fma_rn(-Qd, p.K.pc[0], s1[j + u]);
-            const double d2 = __fma_rn(-Qd, p.K.pc[1], s2[j + u]);
-            const double d3 = __fma_rn(-Qd, p.K.pc[2], s3[j + u]);
-            const double cc = __fma_rn(__fma_rn(d1, 0x1p40, d2), 0x1p40, d3);
-            v[u] = (srow == NONFINITE || scol == NONFINITE) ? __longlong_as_double(0x7ff8000000000000ll)
-                                                            : scale2(cc, p.K.E3 - srow - scol);
-        }
-        const int col = col0 + j;
-        if (col + 1 < p.n && p.vec_store) {
-            double2 *dst = reinterpret_cast<double2 *>(crow + col);
-            if (p.beta_one) {
-                const double2 o = *dst;
-                v[0] = __dadd_rn(o.x, v[0]);
-                v[1] = __dadd_rn(o.y, v[1]);
+    for (int j0 = 0; j0 < 8; j0 += 4) {
+        double s1[4], s2[4], s3[4], v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s1[j] = s2[j] = s3[j] = 0.0;
+#pragma unroll
+        for (int l = 0; l < Q; ++l) {
+            const uint32_t word = j0 == 0 ? res[l].x : res[l].y;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const double r = __hiloint2double((int)__byte_perm(word, 0u, 0x4404 | (j << 4)), 0);  // R 2^-1034
+                s1[j] = __fma_rn(p.K.w[l][0], r, s1[j]);
+                s2[j] = __fma_rn(p.K.w[l][1], r, s2[j]);
+                s3[j] = __fma_rn(p.K.w[l][2], r, s3[j]);
             }
-            *dst = make_double2(v[0], v[1]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const double q = __dmul_rn(__fma_rn(s2[j], 0x1p-40, s1[j]), p.K.inv_phat);
+            const double Qd = __dsub_rn(__dadd_rn(q, kRound), kRound);  // rint(q), |q| < 2^12
+            const double d1 = __fma_rn(-Qd, p.K.pc[0], s1[j]);
+            const double d2 = __fma_rn(-Qd, p.K.pc[1], s2[j]);
+            const double d3 = __fma_rn(-Qd, p.K.pc[2], s3[j]);
+            const double cc = __fma_rn(__fma_rn(d1, 0x1p40, d2), 0x1p40, d3);
+            if (plain) {
+                v[j] = __dmul_rn(cc, __hiloint2double((e[j0 + j] + 1023) << 20, 0));
+            } else {
+                const int scol = p.tu[min(col0 + j0 + j, p.n - 1)];
+                v[j] = (srow == NONFINITE || scol == NONFINITE) ? __longlong_as_double(0x7ff8000000000000ll)
+                                                                : scale2(cc, e[j0 + j]);
+            }
+        }
+        if (p.vec_store == 4) {
+            const int col = col0 + j0;
+            double *dst = p.C + (size_t)row * p.ldc + col;
+            if (row >= p.m) continue;
+            if (col + 3 < p.n) {
+                if (p.beta_one) {
+                    double o[4];
+                    asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
+                                 : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3])
+                                 : "l"(dst));
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) v[u] = __dadd_rn(o[u], v[u]);
+                }
+                asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(dst), "d"(v[0]), "d"(v[1]), "d"(v[2]),
+                             "d"(v[3])
+                             : "memory");
+            } else {
+#pragma unroll
+                for (int u = 0; u < 3; ++u)
+                    if (col + u < p.n) dst[u] = p.beta_one ? __dadd_rn(dst[u], v[u]) : v[u];
+            }
+            continue;
+        }
+        double2 *o = reinterpret_cast<double2 *>(&out[lane][warp * 8 + j0]);
+        o[0] = make_double2(v[0], v[1]);
+        o[1] = make_double2(v[2], v[3]);
+    }
+    if (p.vec_store == 4) return;
+    __syncthreads();
+    // warp w writes rows 4 w ..: 64 columns each
+    const int cbase = tn * TILE + (c & ~7) * 8;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = warp * 4 + i;
+        if (row0 + r >= p.m) break;
+        double *crow = p.C + (size_t)(row0 + r) * p.ldc + cbase;
+        if (p.vec_store) {
+            const int cc = 2 * lane;
+            const double2 v = *reinterpret_cast<const double2 *>(&out[r][cc]);
+            if (cbase + cc + 1 < p.n) {
+                double2 *dst = reinterpret_cast<double2 *>(crow + cc);
+                const double2 o = p.beta_one ? *dst : make_double2(0.0, 0.0);
+                *dst = p.beta_one ? make_double2(__dadd_rn(o.x, v.x), __dadd_rn(o.y, v.y)) : v;
+            } else if (cbase + cc < p.n) {
+                crow[cc] = p.beta_one ? __dadd_rn(crow[cc], v.x) : v.x;
+            }
         } else {
-            if (col < p.n) crow[col] = p.beta_one ? __dadd_rn(crow[col], v[0]) : v[0];
-            if (col + 1 < p.n) crow[col + 1] = p.beta_one ? __dadd_rn(crow[col + 1], v[1]) : v[1];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int cc = lane + 32 * u;
+                if (cbase + cc < p.n) crow[cc] = p.beta_one ? __dadd_rn(crow[cc], out[r][cc]) : out[r][cc];
+            }
         }
     }
 }
@@ -826,7 +904,7 @@ static bool make_consts(int q, Consts &K)
     K.L = L;
     K.alpha = (L - 3) / 2;
     K.beta = L - 3 - K.alpha;
-    K.E3 = L - 120;
+    K.E3 = L - 120 + kCombineShift;
     for (int l = 0; l < q; ++l) {
         const unsigned p = (unsigned)h_moduli[l];
         const unsigned __int128 M = P / p;
@@ -834,12 +912,14 @@ static bool make_consts(int q, Consts &K)
         unsigned inv = 1;
         while ((mm * inv) % p != 1) ++inv;
         chunks40(M * inv, L, K.w[l]);
+        for (double &c : K.w[l]) c = ldexp(c, 1034 - kCombineShift);
         K.c32[l] = (double)((1ull << 32) % p);
         K.inv_p[l] = 1.0 / (double)p;
         K.barrett[l] = (uint32_t)(0xffffffffull / p + 1);
     }
     chunks40(P, L, K.pc);
-    K.inv_phat = 1.0 / fma(K.pc[1], 0x1p-40, K.pc[0]);
+    K.inv_phat = ldexp(1.0 / fma(K.pc[1], 0x1p-40, K.pc[0]), kCombineShift);
+    for (double &c : K.pc) c = ldexp(c, -kCombineShift);
     return true;
 }
 
@@ -946,13 +1026,12 @@ struct SplitB {
 
 template <int Q>
 struct Combine {
-    static int run(const crt::CombineParams &cp, long long units, cudaStream_t stream)
+    static int run(const crt::CombineParams &cp, long long blocks, cudaStream_t stream)
     {
-        const long long blocks = (units + 7) / 8;
         if (cp.ksplit > 1)
-            crt::crt_combine<Q, true><<<(unsigned)blocks, 256, 0, stream>>>(cp, units);
+            crt::crt_combine<Q, true><<<(unsigned)blocks, 256, 0, stream>>>(cp);
         else
-            crt::crt_combine<Q, false><<<(unsigned)blocks, 256, 0, stream>>>(cp, units);
+            crt::crt_combine<Q, false><<<(unsigned)blocks, 256, 0, stream>>>(cp);
         MGX_HOST_CHECK(cudaGetLastError());
         return MGX_SUCCESS;
     }
@@ -1091,13 +1170,16 @@ int crt_combine_impl(double *C, int ldc, int beta_one, const crt::Consts &K, con
     cp.tiles_n = v.tiles_n;
     cp.rc_tile_ld = L.tiles_n;
     cp.beta_one = beta_one;
-    cp.vec_store = ((ldc & 1) == 0) && ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
+    // doubles that C's rows are aligned to: 4, 2 or (0) one
+    cp.vec_store = (ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 31) == 0)   ? 4
+                   : (ldc % 2 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) ? 2
+                                                                                  : 0;
     cp.sg = v.sg;
     cp.tu = v.tu;
     cp.K = K;
-    const long long units = (long long)v.tiles_m * v.tiles_n * 256;
-    if (units <= 0) return MGX_SUCCESS;
-    return dispatch_q<Combine>(K.q, cp, units, stream);
+    const long long blocks = (long long)v.tiles_m * v.tiles_n * 32;
+    if (blocks <= 0) return MGX_SUCCESS;
+    return dispatch_q<Combine>(K.q, cp, blocks, stream);
 }
 
 int crt_multiply_impl(double *C, int m, int n, int ldc, int beta_one, const crt::Consts &K, unsigned char *ws,
