@@ -305,8 +305,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     // Launched as a programmatic dependent: everything above overlapped the previous kernel in the
     // stream; nothing below reads or writes memory before that kernel has finished.  The next
     // kernel may be scheduled now (it cannot share an SM with this one, and waits the same way).
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_wait();
+    pdl_trigger();
 
     Walk walk;
     walk.init(p);
@@ -790,20 +790,9 @@ static int launch_dgemm(const double *A, const double *B, double *C, int m, int 
             return MGX_E_UNSUPPORTED;
         }
         MGX_HOST_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fp64::SMEM_BYTES));
-        // programmatic dependent launch: the set-up above griddepcontrol.wait overlaps the end of
-        // the previous kernel in the stream
-        cudaLaunchConfig_t cfg;
-        memset(&cfg, 0, sizeof cfg);
-        cfg.gridDim = dim3((unsigned)grid);
-        cfg.blockDim = dim3(fp64::THREADS);
-        cfg.dynamicSmemBytes = (size_t)fp64::SMEM_BYTES;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        MGX_HOST_CHECK(cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, p));
+        // the set-up above the kernel's wait overlaps the end of the previous kernel in the stream
+        MGX_HOST_CHECK(mgx_launch_dependent(kernel, dim3((unsigned)grid), dim3(fp64::THREADS), fp64::SMEM_BYTES, stream,
+                                            tmA, tmB, p));
         return MGX_SUCCESS;
     };
     if (rc == MGX_SUCCESS) rc = panels ? launch(fp64::dgemm_kernel<true>) : launch(fp64::dgemm_kernel<false>);

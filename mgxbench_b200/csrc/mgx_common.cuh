@@ -37,7 +37,29 @@ int mgx_encode_tmap_3d(CUtensorMap *map, CUtensorMapDataType dtype, int elem_byt
                        uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1_bytes, uint64_t stride2_bytes,
                        uint32_t b0, uint32_t b1, uint32_t b2, CUtensorMapSwizzle swizzle);
 
+// Programmatic dependent launch: the kernel may be scheduled while the one before it in the stream
+// drains.  It must execute pdl_wait() before it touches memory; pdl_trigger() lets the next one in.
+template <typename... Params, typename... Args>
+static inline cudaError_t mgx_launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                                               cudaStream_t stream, const Args &...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 namespace mgx {
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Device status codes (first error wins).
 enum DeviceStatus : int {

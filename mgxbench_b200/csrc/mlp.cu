@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(THREADS) forward_kernel(const float *__restric
                                                           const float *__restrict__ params, float *__restrict__ out)
 {
     __shared__ Net n;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_wait();
     load_params(n, params);
     for (int s0 = blockIdx.x * SPB; s0 < batch; s0 += gridDim.x * SPB) {
         const int ns = min(SPB, batch - s0);
@@ -138,8 +138,8 @@ __global__ void __launch_bounds__(THREADS) forward_kernel(const float *__restric
 // it has finished, so that kernel may read its inputs before its own wait.
 __global__ void __launch_bounds__(THREADS) zero_kernel(float *__restrict__ grads, float *__restrict__ loss)
 {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * THREADS + threadIdx.x;
     if (i < NPARAM) grads[i] = 0.f;
     if (i == NPARAM) *loss = 0.f;
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(THREADS) grad_kernel(const float *__restrict__
             }
     }
     __syncthreads();
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // grads and loss are zero from here on
+    pdl_wait();  // grads and loss are zero from here on
     if (t == 0) atomicAdd(loss, lpart);
 #pragma unroll
     for (int a = 0; a < 4; ++a)
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(THREADS) grad_kernel(const float *__restrict__
 __global__ void adam_kernel(float *__restrict__ params, const float *__restrict__ grads, float *__restrict__ m,
                             float *__restrict__ v, int step, float lr, float beta1, float beta2, float eps)
 {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= NPARAM) return;
     const float g = grads[i];
@@ -302,21 +302,10 @@ __global__ void init_kernel(float *__restrict__ params, unsigned long long seed)
 
 using namespace mgx;
 
-// Programmatic dependent launch: the kernel may be scheduled while the one before it in the stream
-// drains; it waits for it (griddepcontrol.wait) before it touches memory.
 template <typename... Params, typename... Args>
-static cudaError_t launch_dependent(void (*kernel)(Params...), int grid, cudaStream_t stream, Args... args)
+static cudaError_t launch_dependent(void (*kernel)(Params...), int grid, cudaStream_t stream, const Args &...args)
 {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(mlp::THREADS);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
+    return mgx_launch_dependent(kernel, dim3((unsigned)grid), dim3(mlp::THREADS), 0, stream, args...);
 }
 
 extern "C" {

@@ -23,7 +23,8 @@
 //
 // Kernels:
 //   crt_row_scale   sigma per row of A (one block per row, integer sum of squares)
-//   crt_col_max / crt_col_sumsq / crt_col_scale   tau per column of B (integer atomics)
+//   crt_col_max / crt_col_sumsq   tau per column of B (integer atomics; the last block of a column
+//                   group takes the scales)
 //   crt_split_a     residues of A as swizzled K-major 256-row slabs [modulus][tile][K block]
 //   crt_split_b     residues of B^T, same layout (thread per column, coalesced reads)
 //   crt_gemm        persistent tcgen05 kernel over (modulus, 256 x 256 tile) work items:
@@ -154,42 +155,79 @@ __device__ __forceinline__ int sigma_of(unsigned long long mx, unsigned long lon
 }
 
 // ---------------------------------------------------------------- scale kernels
-// One block of ROW_THREADS per row: the row's maximum, then its integer sum of squares.  The
-// second pass finds the row in L2: at 4 blocks per SM, 592 rows (77 MB at k = 16384) are in
-// flight, against L2's 126 MB, so A is read from DRAM once.
-constexpr int ROW_THREADS = 512;
+// What the column passes add to and count with, zeroed before them: by the row pass of the same
+// split, or by crt_zero.
+struct ColStats {
+    unsigned long long *max, *sum;  // per column
+    unsigned int *arrived;          // per group of 256 columns: blocks of crt_col_sumsq that are done
+    int n;
+};
 
-__global__ void __launch_bounds__(ROW_THREADS) crt_row_scale(const double *__restrict__ A, int m, int k, int lda,
-                                                             int target, int *__restrict__ sg, int *status)
+__device__ __forceinline__ void zero_stats(const ColStats &z, long long i, long long step)
 {
-    __shared__ unsigned long long red[ROW_THREADS / 32];
-    __shared__ unsigned long long row_max;
-    const int row = blockIdx.x;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (row >= m) return;
+    for (; i < z.n; i += step) {
+        z.max[i] = 0ull;
+        z.sum[i] = 0ull;
+        if (i % 256 == 0) z.arrived[i / 256] = 0u;
+    }
+}
+
+__global__ void __launch_bounds__(256) crt_zero(const ColStats z)
+{
+    pdl_wait();
+    pdl_trigger();
+    zero_stats(z, blockIdx.x * 256 + threadIdx.x, gridDim.x * 256ll);
+}
+
+// Maximum over a warp of non-negative doubles' bit patterns, as far as the scale needs it: the high
+// words' maximum, and the low words' only where no high word is set (the exponent of a value with a
+// non-zero high word does not depend on its low word, nor do the zero and non-finite tests).
+__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v)
+{
+    const uint32_t hi = __reduce_max_sync(0xffffffffu, (uint32_t)(v >> 32));
+    if (hi != 0) return (unsigned long long)hi << 32;
+    return __reduce_max_sync(0xffffffffu, (uint32_t)v);
+}
+
+// One block of T threads per row: the row's maximum, then its integer sum of squares.
+// KEEP > 0: rows of at most KEEP x T elements, held in registers, so A is read once and the loads of a
+// row are all in flight together.  Longer rows (KEEP = 0, 512 threads): the second pass finds
+// the row in L2 (at 4 blocks per SM, 592 rows, 77 MB at k = 16384, are in flight, against L2's 126 MB),
+// so A is read from DRAM once there too.  With 512 threads and two passes for every row, 2501 rows of
+// 3001 took 25 us, mostly waiting on a few short loads per thread; now 16.
+template <int T, int KEEP>
+__global__ void __launch_bounds__(T) crt_row_scale(const double *__restrict__ A, int m, int k, int lda, int target,
+                                                   int *__restrict__ sg, const ColStats z, int *status)
+{
+    __shared__ unsigned long long red[T / 32], sum[T / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = blockIdx.x;
+    pdl_wait();
+    pdl_trigger();
+    zero_stats(z, (long long)blockIdx.x * T + threadIdx.x, (long long)gridDim.x * T);
     const double *r = A + (size_t)row * lda;
-    const unsigned long long *rb = reinterpret_cast<const unsigned long long *>(r);
     unsigned long long mx = 0;
-    for (int kk = threadIdx.x; kk < k; kk += ROW_THREADS) {
-        const unsigned long long b = __ldg(rb + kk) & 0x7fffffffffffffffull;
-        mx = b > mx ? b : mx;
+    double v[KEEP > 0 ? KEEP : 1];
+    if constexpr (KEEP > 0) {
+#pragma unroll
+        for (int u = 0; u < KEEP; ++u) {
+            const int kk = threadIdx.x + u * T;
+            v[u] = kk < k ? __ldg(r + kk) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < KEEP; ++u) {
+            const unsigned long long b = (unsigned long long)__double_as_longlong(v[u]) & 0x7fffffffffffffffull;
+            mx = b > mx ? b : mx;
+        }
+    } else {
+        for (int kk = threadIdx.x; kk < k; kk += T) {
+            const unsigned long long b = (unsigned long long)__double_as_longlong(__ldg(r + kk)) & 0x7fffffffffffffffull;
+            mx = b > mx ? b : mx;
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long other = __shfl_xor_sync(0xffffffffu, mx, o);
-        mx = other > mx ? other : mx;
-    }
+    mx = warp_max_bits(mx);
     if (lane == 0) red[warp] = mx;
     __syncthreads();
-    if (warp == 0) {
-        mx = lane < ROW_THREADS / 32 ? red[lane] : 0ull;
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long other = __shfl_xor_sync(0xffffffffu, mx, o);
-            mx = other > mx ? other : mx;
-        }
-        if (lane == 0) row_max = mx;
-    }
-    __syncthreads();
-    mx = row_max;
+    mx = warp_max_bits(lane < T / 32 ? red[lane] : 0ull);
     if (mx >= 0x7ff0000000000000ull) {
         if (threadIdx.x == 0) {
             sg[row] = NONFINITE;
@@ -202,80 +240,98 @@ __global__ void __launch_bounds__(ROW_THREADS) crt_row_scale(const double *__res
     scale_factors(22 - e, f1, f2);
     unsigned long long S = 0;  // an exact integer sum: the order of its terms does not matter
     if (mx != 0) {
-        int kk = threadIdx.x;
-        for (; kk + 3 * ROW_THREADS < k; kk += 4 * ROW_THREADS) {
-            double v[4];
+        if constexpr (KEEP > 0) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = __ldg(r + kk + u * ROW_THREADS);
+            for (int u = 0; u < KEEP; ++u) S += sq_term(v[u], f1, f2);
+        } else {
+            int kk = threadIdx.x;
+            for (; kk + 3 * T < k; kk += 4 * T) {
+                double w[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) S += sq_term(v[u], f1, f2);
+                for (int u = 0; u < 4; ++u) w[u] = __ldg(r + kk + u * T);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) S += sq_term(w[u], f1, f2);
+            }
+            for (; kk < k; kk += T) S += sq_term(__ldg(r + kk), f1, f2);
         }
-        for (; kk < k; kk += ROW_THREADS) S += sq_term(__ldg(r + kk), f1, f2);
     }
     for (int o = 16; o > 0; o >>= 1) S += __shfl_xor_sync(0xffffffffu, S, o);
-    if (lane == 0) red[warp] = S;   // warp 0 read red[] before the barrier above
+    if (lane == 0) sum[warp] = S;
     __syncthreads();
     if (warp == 0) {
-        S = lane < ROW_THREADS / 32 ? red[lane] : 0ull;
-        for (int o = 16; o > 0; o >>= 1) S += __shfl_xor_sync(0xffffffffu, S, o);
+        S = lane < T / 32 ? sum[lane] : 0ull;
+        for (int o = T / 64; o > 0; o >>= 1) S += __shfl_xor_sync(0xffffffffu, S, o);
         if (lane == 0) sg[row] = sigma_of(mx, S, target);
     }
 }
 
-// grid (ceil(n/256), ychunks); each thread scans a run of rows of one column.
-__global__ void crt_col_max(const double *__restrict__ B, int k, int n, int ldb, unsigned long long *colmax)
+// grid (ceil(n/256), ychunks); each thread scans a run of rows of one column, 8 loads in flight.
+__global__ void __launch_bounds__(256) crt_col_max(const double *__restrict__ B, int k, int n, int ldb,
+                                                   unsigned long long *colmax)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
+    const int j = blockIdx.x * 256 + threadIdx.x;
     if (j >= n) return;
     const int rows_per = (k + gridDim.y - 1) / gridDim.y;
     const int r0 = blockIdx.y * rows_per;
     const int r1 = min(k, r0 + rows_per);
     unsigned long long mx = 0;
-    const unsigned long long *b = reinterpret_cast<const unsigned long long *>(B);
-    for (int r = r0; r < r1; ++r) {
-        const unsigned long long v = __ldg(b + (size_t)r * ldb + j) & 0x7fffffffffffffffull;
+    const unsigned long long *b = reinterpret_cast<const unsigned long long *>(B) + j;
+    int r = r0;
+    for (; r + 8 <= r1; r += 8) {
+        unsigned long long v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = __ldg(b + (size_t)(r + u) * ldb) & 0x7fffffffffffffffull;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) mx = v[u] > mx ? v[u] : mx;
+    }
+    for (; r < r1; ++r) {
+        const unsigned long long v = __ldg(b + (size_t)r * ldb) & 0x7fffffffffffffffull;
         mx = v > mx ? v : mx;
     }
     if (mx) atomicMax(colmax + j, mx);
 }
 
-__global__ void crt_col_sumsq(const double *__restrict__ B, int k, int n, int ldb,
-                              const unsigned long long *__restrict__ colmax, unsigned long long *colsum)
+// The same grid: sums of squares, then tau, taken by the last block of each column group to arrive.
+__global__ void __launch_bounds__(256) crt_col_sumsq(const double *__restrict__ B, int k, int n, int ldb,
+                                                     const ColStats z, int target, int *__restrict__ tu, int *status)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const unsigned long long mx = colmax[j];
-    if (mx == 0 || mx >= 0x7ff0000000000000ull) return;
-    const int e = frexp_exp_bits(mx);
-    double f1, f2;
-    scale_factors(22 - e, f1, f2);
-    const int rows_per = (k + gridDim.y - 1) / gridDim.y;
-    const int r0 = blockIdx.y * rows_per;
-    const int r1 = min(k, r0 + rows_per);
-    unsigned long long S = 0;  // an exact integer sum: the order of its terms does not matter
-    int r = r0;
-    for (; r + 8 <= r1; r += 8) {
-        double v[8];
+    __shared__ bool last;
+    pdl_wait();
+    pdl_trigger();
+    const int j = blockIdx.x * 256 + threadIdx.x;
+    const unsigned long long mx = j < n ? z.max[j] : 0ull;
+    if (mx != 0 && mx < 0x7ff0000000000000ull) {
+        const int e = frexp_exp_bits(mx);
+        double f1, f2;
+        scale_factors(22 - e, f1, f2);
+        const int rows_per = (k + gridDim.y - 1) / gridDim.y;
+        const int r0 = blockIdx.y * rows_per;
+        const int r1 = min(k, r0 + rows_per);
+        unsigned long long S = 0;  // an exact integer sum: the order of its terms does not matter
+        int r = r0;
+        for (; r + 8 <= r1; r += 8) {
+            double v[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = __ldg(B + (size_t)(r + u) * ldb + j);
+            for (int u = 0; u < 8; ++u) v[u] = __ldg(B + (size_t)(r + u) * ldb + j);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) S += sq_term(v[u], f1, f2);
+            for (int u = 0; u < 8; ++u) S += sq_term(v[u], f1, f2);
+        }
+        for (; r < r1; ++r) S += sq_term(__ldg(B + (size_t)r * ldb + j), f1, f2);
+        if (S) atomicAdd(z.sum + j, S);
     }
-    for (; r < r1; ++r) S += sq_term(__ldg(B + (size_t)r * ldb + j), f1, f2);
-    if (S) atomicAdd(colsum + j, S);
-}
-
-__global__ void crt_col_scale(const unsigned long long *__restrict__ colmax, const unsigned long long *__restrict__ colsum,
-                              int n, int target, int *__restrict__ tu, int *status)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const unsigned long long mx = colmax[j];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(z.arrived + blockIdx.x, 1u) == gridDim.y - 1;
+    __syncthreads();
+    if (!last || j >= n) return;
+    __threadfence();
     if (mx >= 0x7ff0000000000000ull) {
         tu[j] = NONFINITE;
         record_status(status, kDevNonFinite);
     } else {
-        tu[j] = sigma_of(mx, colsum[j], target);
+        tu[j] = sigma_of(mx, __ldcg(z.sum + j), target);
     }
 }
 
@@ -343,6 +399,8 @@ __global__ void __launch_bounds__(256, 3) crt_split_a(const double *__restrict__
                                                       int kblocks, const int *__restrict__ sg, uint8_t *__restrict__ ra,
                                                       size_t mod_stride, const __grid_constant__ Consts K)
 {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int kb = blockIdx.y;
     const int row = blockIdx.x * 64 + warp * 8 + (lane >> 2), kq = lane & 3;
@@ -380,6 +438,8 @@ __global__ void __launch_bounds__(256, 3) crt_split_b(const double *__restrict__
                                                       size_t mod_stride, const __grid_constant__ Consts K)
 {
     __shared__ __align__(16) unsigned char st[Q][64 * 32];
+    pdl_wait();
+    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kb = blockIdx.y, kq = warp & 3;
     const int rl = (warp >> 2) * 32 + lane;          // row of the block's 64
@@ -553,6 +613,8 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();  // the set-up above overlaps the end of the previous kernel
+    pdl_trigger();
 
     if (warp == 0) {
         // ------------------------------------------------------------ bulk-copy producer
@@ -744,6 +806,8 @@ __global__ void __launch_bounds__(256, SPLITK ? 2 : 3) crt_combine(const __grid_
 {
     const int lane = threadIdx.x & 31;
     __shared__ __align__(16) double out[32][COMBINE_LD];
+    pdl_wait();
+    pdl_trigger();
     const int warp = threadIdx.x >> 5;
     const long long unit = (long long)blockIdx.x * 8 + warp;
     const int c = (int)(unit & 31), qd = (int)((unit >> 5) & 3), h = (int)((unit >> 7) & 1);
@@ -933,7 +997,7 @@ namespace {
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 struct CrtLayout {
-    size_t ra, rb, rc, sg, tu, colmax, colsum, sync, total;
+    size_t ra, rb, rc, sg, tu, colmax, colsum, sync, arrived, total;
     size_t ra_mod, rb_mod, rc_mod;
     int kblocks, tiles_m, tiles_n;
     int ksplit, kb_split;   // K slices (1: whole K) and K blocks per slice
@@ -975,6 +1039,8 @@ CrtLayout crt_layout(int m, int n, int k, int q, int ksplit = 1)
     off = align256(off + sizeof(unsigned long long) * (size_t)n);
     L.sync = off;                       // arrival counters of the products launches (two slots)
     off = align256(off + 2 * sizeof(unsigned int));
+    L.arrived = off;                    // per column group: blocks that are done with its sums
+    off = align256(off + sizeof(unsigned int) * (size_t)((n + 255) / 256));
     L.total = off;
     return L;
 }
@@ -1004,9 +1070,8 @@ struct SplitA {
                    const crt::Consts &K, cudaStream_t stream)
     {
         const int tiles = (m + crt::TILE - 1) / crt::TILE;
-        crt::crt_split_a<Q><<<dim3(tiles * 4, L.kblocks), 256, 0, stream>>>(A, m, k, lda, tiles * crt::TILE,
-                                                                            L.kblocks, sg, ra, L.ra_mod, K);
-        MGX_HOST_CHECK(cudaGetLastError());
+        MGX_HOST_CHECK(mgx_launch_dependent(crt::crt_split_a<Q>, dim3(tiles * 4, L.kblocks), 256, 0, stream, A, m, k, lda,
+                                            tiles * crt::TILE, L.kblocks, sg, ra, L.ra_mod, K));
         return MGX_SUCCESS;
     }
 };
@@ -1017,9 +1082,8 @@ struct SplitB {
                    const crt::Consts &K, cudaStream_t stream)
     {
         const int tiles = (n + crt::TILE - 1) / crt::TILE;
-        crt::crt_split_b<Q><<<dim3(tiles * 4, L.kblocks), 256, 0, stream>>>(B, k, n, ldb, L.kblocks, tu, rb, L.rb_mod,
-                                                                            K);
-        MGX_HOST_CHECK(cudaGetLastError());
+        MGX_HOST_CHECK(mgx_launch_dependent(crt::crt_split_b<Q>, dim3(tiles * 4, L.kblocks), 256, 0, stream, B, k, n, ldb,
+                                            L.kblocks, tu, rb, L.rb_mod, K));
         return MGX_SUCCESS;
     }
 };
@@ -1028,59 +1092,71 @@ template <int Q>
 struct Combine {
     static int run(const crt::CombineParams &cp, long long blocks, cudaStream_t stream)
     {
-        if (cp.ksplit > 1)
-            crt::crt_combine<Q, true><<<(unsigned)blocks, 256, 0, stream>>>(cp);
-        else
-            crt::crt_combine<Q, false><<<(unsigned)blocks, 256, 0, stream>>>(cp);
-        MGX_HOST_CHECK(cudaGetLastError());
+        MGX_HOST_CHECK(mgx_launch_dependent(cp.ksplit > 1 ? crt::crt_combine<Q, true> : crt::crt_combine<Q, false>,
+                                            dim3((unsigned)blocks), 256, 0, stream, cp));
         return MGX_SUCCESS;
     }
 };
 
+crt::ColStats col_stats(unsigned char *ws, const CrtLayout &L, int c0, int n)
+{
+    crt::ColStats z;
+    z.max = reinterpret_cast<unsigned long long *>(ws + L.colmax) + c0;
+    z.sum = reinterpret_cast<unsigned long long *>(ws + L.colsum) + c0;
+    z.arrived = reinterpret_cast<unsigned int *>(ws + L.arrived) + c0 / 256;
+    z.n = n;
+    return z;
+}
+
 // Scale exponents and residues of rows [r0, r0 + m) of A (m x k, k <= KMAX; r0 a multiple of
-// 256) into the whole-problem workspace.
+// 256) into the whole-problem workspace.  `zero`: column statistics for the row pass to clear.
 int crt_split_a_impl(const double *A, int m, int k, int lda, int r0, const crt::Consts &K, unsigned char *ws,
-                     const CrtLayout &L, cudaStream_t stream)
+                     const CrtLayout &L, cudaStream_t stream, const crt::ColStats &zero = crt::ColStats{})
 {
     if (m <= 0) return MGX_SUCCESS;
     int *status = mgx_device_status_ptr();
     int *sg = reinterpret_cast<int *>(ws + L.sg) + r0;
     uint8_t *ra = ws + L.ra + (size_t)(r0 / crt::TILE) * L.kblocks * crt::SLAB;
-    crt::crt_row_scale<<<m, crt::ROW_THREADS, 0, stream>>>(A, m, k, lda, K.alpha, sg, status);
-    MGX_HOST_CHECK(cudaGetLastError());
+    // the fewest threads that hold a row in 16 registers each
+    auto scale = [&](auto kernel, int threads) {
+        return mgx_launch_dependent(kernel, dim3((unsigned)m), dim3(threads), 0, stream, A, m, k, lda, K.alpha, sg, zero,
+                                    status);
+    };
+    MGX_HOST_CHECK(k <= 1024   ? scale(crt::crt_row_scale<64, 16>, 64)
+                   : k <= 2048 ? scale(crt::crt_row_scale<128, 16>, 128)
+                   : k <= 4096 ? scale(crt::crt_row_scale<256, 16>, 256)
+                   : k <= 8192 ? scale(crt::crt_row_scale<512, 16>, 512)
+                               : scale(crt::crt_row_scale<512, 0>, 512));
     return dispatch_q<SplitA>(K.q, A, m, k, lda, L, (const int *)sg, ra, K, stream);
 }
 
-// The same for columns [c0, c0 + n) of B (k x n).
+// The same for columns [c0, c0 + n) of B (k x n).  `zeroed`: their statistics are clear.
 int crt_split_b_impl(const double *B, int n, int k, int ldb, int c0, const crt::Consts &K, unsigned char *ws,
-                     const CrtLayout &L, cudaStream_t stream)
+                     const CrtLayout &L, cudaStream_t stream, bool zeroed = false)
 {
     if (n <= 0) return MGX_SUCCESS;
     int *status = mgx_device_status_ptr();
     int *tu = reinterpret_cast<int *>(ws + L.tu) + c0;
-    unsigned long long *colmax = reinterpret_cast<unsigned long long *>(ws + L.colmax) + c0;
-    unsigned long long *colsum = reinterpret_cast<unsigned long long *>(ws + L.colsum) + c0;
+    const crt::ColStats z = col_stats(ws, L, c0, n);
     uint8_t *rb = ws + L.rb + (size_t)(c0 / crt::TILE) * L.kblocks * crt::SLAB;
-    MGX_HOST_CHECK(cudaMemsetAsync(colmax, 0, sizeof(unsigned long long) * (size_t)n, stream));
-    MGX_HOST_CHECK(cudaMemsetAsync(colsum, 0, sizeof(unsigned long long) * (size_t)n, stream));
+    const int groups = (n + 255) / 256;
+    if (!zeroed)
+        MGX_HOST_CHECK(mgx_launch_dependent(crt::crt_zero, dim3((unsigned)(groups < 64 ? groups : 64)), 256, 0, stream, z));
     const int sms = mgx_sm_count();
-    int ych = (sms * 8) / ((n + 255) / 256);
+    int ych = (sms * 8) / groups;
     if (ych > (k + 63) / 64) ych = (k + 63) / 64;
     if (ych < 1) ych = 1;
-    crt::crt_col_max<<<dim3((n + 255) / 256, ych), 256, 0, stream>>>(B, k, n, ldb, colmax);
-    MGX_HOST_CHECK(cudaGetLastError());
-    crt::crt_col_sumsq<<<dim3((n + 255) / 256, ych), 256, 0, stream>>>(B, k, n, ldb, colmax, colsum);
-    MGX_HOST_CHECK(cudaGetLastError());
-    crt::crt_col_scale<<<(n + 255) / 256, 256, 0, stream>>>(colmax, colsum, n, K.beta, tu, status);
-    MGX_HOST_CHECK(cudaGetLastError());
+    const dim3 grid((unsigned)groups, (unsigned)ych);
+    MGX_HOST_CHECK(mgx_launch_dependent(crt::crt_col_max, grid, 256, 0, stream, B, k, n, ldb, z.max));
+    MGX_HOST_CHECK(mgx_launch_dependent(crt::crt_col_sumsq, grid, 256, 0, stream, B, k, n, ldb, z, K.beta, tu, status));
     return dispatch_q<SplitB>(K.q, B, n, k, ldb, L, (const int *)tu, rb, K, stream);
 }
 
 int crt_split_impl(const double *A, const double *B, int m, int n, int k, int lda, int ldb, const crt::Consts &K,
                    unsigned char *ws, const CrtLayout &L, cudaStream_t stream)
 {
-    int rc = crt_split_a_impl(A, m, k, lda, 0, K, ws, L, stream);
-    if (rc == MGX_SUCCESS) rc = crt_split_b_impl(B, n, k, ldb, 0, K, ws, L, stream);
+    int rc = crt_split_a_impl(A, m, k, lda, 0, K, ws, L, stream, col_stats(ws, L, 0, n));
+    if (rc == MGX_SUCCESS) rc = crt_split_b_impl(B, n, k, ldb, 0, K, ws, L, stream, true);
     return rc;
 }
 
@@ -1143,13 +1219,16 @@ int crt_products_impl(const crt::Consts &K, const CrtLayout &L, const CrtView &v
     }
     const int sms = mgx_sm_count();
     const int grid = (long long)sms < items ? sms : (int)items;
-    if (sync) {
+    // The lockstep pays over many items (8192 x 8192 x 1024, 104 per CTA: 1.57 ms with it, 1.60 without;
+    // 3000 x 3000 x 16384, 15: 2.46, 2.59).  Over few, its counter's memset, which also keeps the products
+    // from being a dependent launch, costs more: 1024^3, 2 per CTA: 68 us with it, 63 without; 2501 x
+    // 1999 x 3001, 8: 344, 340.
+    if (sync && items >= 10ll * grid) {
         MGX_HOST_CHECK(cudaMemsetAsync(sync, 0, sizeof(unsigned int), stream));
         p.sync = sync;
     }
     MGX_HOST_CHECK(cudaFuncSetAttribute(crt::crt_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    crt::crt_gemm<<<grid, crt::THREADS, smem, stream>>>(p);
-    MGX_HOST_CHECK(cudaGetLastError());
+    MGX_HOST_CHECK(mgx_launch_dependent(crt::crt_gemm, dim3((unsigned)grid), crt::THREADS, smem, stream, p));
     return MGX_SUCCESS;
 }
 
