@@ -33,9 +33,11 @@
 //                   the CTAs that share an operand tile read it within microseconds of each
 //                   other and mostly from L2 (DRAM reads at N = 16384: 118 -> 48 GB per launch)
 //       warp 1      TMEM owner and MMA issuer: two M=128 N=256 K=32 kind::i8 MMAs per K block
-//                   (rows 0-127 and 128-255), int32 accumulators in all 512 TMEM columns
-//       warps 2-17  epilogue (16 warps, two per accumulator and TMEM lane quarter, 128 columns
-//                   each): tcgen05.ld, exact reduction mod p_l (biased Barrett), one byte per output
+//                   (rows 0-127 and 128-255), int32 accumulators in all 512 TMEM columns, each
+//                   handed over on its own
+//       warps 2-17  epilogue (16 warps, four per TMEM lane quarter, 64 columns each): both
+//                   accumulators in turn: tcgen05.ld, release, exact reduction mod p_l (biased
+//                   Barrett), one byte per output
 //   crt_combine     CRT recombination of the q residue planes, scaling, (C +) store
 // All waits are bounded (mgx_common.cuh); TMEM is always released before the CTA exits.
 #include <cmath>
@@ -63,13 +65,7 @@ constexpr int SLAB = TILE * KB;        // 8 KiB: one operand, one K block
 constexpr int KPACK = MGX_CRT_KPACK;   // K blocks per pipeline stage
 constexpr int STAGE_BYTES = 2 * KPACK * SLAB;
 constexpr int STAGES = (232448 - 1280) / STAGE_BYTES;   // 227 KiB of shared memory per CTA
-#ifndef MGX_CRT_EPI_WARPS
-#define MGX_CRT_EPI_WARPS 16
-#endif
-constexpr int EPI_WARPS = MGX_CRT_EPI_WARPS;   // 8 or 16: one or two warps per (accumulator, TMEM lane quarter)
-constexpr int COL_SPLIT = EPI_WARPS / 8;       // warps sharing the 256 columns of one accumulator's lane quarter
-constexpr int EPI_CHUNKS = 8 / COL_SPLIT;      // 32-column chunks each epilogue warp drains
-static_assert(EPI_WARPS == 8 || EPI_WARPS == 16, "epilogue warps");
+constexpr int EPI_WARPS = 16;          // four per TMEM lane quarter, 64 columns of either accumulator each
 constexpr int THREADS = (2 + EPI_WARPS) * 32;
 constexpr int NONFINITE = 0x7fffffff;
 constexpr int OUT_TILE_BYTES = TILE * TILE;   // one residue byte per output
@@ -585,9 +581,9 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
                                                             ~uintptr_t(1023));
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES);
     uint64_t *empty = full + STAGES;
-    uint64_t *acc_full = empty + STAGES;
-    uint64_t *acc_empty = acc_full + 1;
-    uint64_t *drain = acc_empty + 1;
+    uint64_t *acc_full = empty + STAGES;   // one per accumulator (tile rows 0-127, 128-255)
+    uint64_t *acc_empty = acc_full + 2;
+    uint64_t *drain = acc_empty + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -598,8 +594,10 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
-        mbar_init(acc_full, 1);
-        mbar_init(acc_empty, EPI_WARPS);
+        for (int h = 0; h < 2; ++h) {
+            mbar_init(&acc_full[h], 1);
+            mbar_init(&acc_empty[h], EPI_WARPS);
+        }
         mbar_init(drain, 1);
         fence_barrier_init();
     }
@@ -669,45 +667,85 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
+        // The epilogue releases accumulator 0 as soon as it has read it and accumulator 1 half a drain
+        // later.  Until then the issuer runs ahead with accumulator 0's MMAs over the stages that are
+        // in shared memory, then catches up with accumulator 1's.  From there on the two MMAs of a K block
+        // follow each other: they share its B tile, and issuing a stage's four MMAs of one
+        // accumulator before the other's costs power (16384^3: 54.3 ms against 51.7).  Against one
+        // hand-over of both accumulators after the whole drain (5,000 idle of 33,800 cycles per item at
+        // K = 3008): 8192 x 8192 x 1024 1.60 -> 1.49 ms, 4096^3 1.14 -> 1.12, 16384^3 51.2 -> 50.8.
         if (lane == 0) {
             int stage = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
             const uint32_t smem_base = smem_u32(smem);
             for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
-                if (!mbar_wait_bounded(acc_empty, acc_phase ^ 1u, p.status, kDevTimeoutAcc)) {
-                    ok = false;
-                    break;
+                const int kb_begin = (w % p.ksplit) * p.kb_split, kb_end = min(p.kblocks, kb_begin + p.kb_split);
+                // MMAs over the stage at `st` that starts at K block kb, of accumulators h0 .. h1
+                auto issue = [&](int st, int kb, bool lo, bool hi) {
+                    const int nkb = min(KPACK, kb_end - kb);
+                    const uint32_t sa = smem_base + st * STAGE_BYTES;
+                    const uint64_t a0 = sw32_desc(sa), b0 = sw32_desc(sa + KPACK * SLAB);
+#pragma unroll
+                    for (int j = 0; j < KPACK; ++j) {
+                        if (j < nkb) {
+                            const uint32_t acc = (kb + j > kb_begin) ? 1u : 0u;
+                            const uint64_t bj = b0 + (uint64_t)((j * SLAB) >> 4);
+                            if (lo) tc_mma_i8(tmem_base, a0 + (uint64_t)((j * SLAB) >> 4), bj, IDESC_S8_128x256, acc);
+                            if (hi)
+                                tc_mma_i8(tmem_base + 256, a0 + (uint64_t)((j * SLAB + SLAB / 2) >> 4), bj,
+                                          IDESC_S8_128x256, acc);
+                        }
+                    }
+                };
+                auto next = [&](int &st, uint32_t &ph) {
+                    if (++st == STAGES) {
+                        st = 0;
+                        ph ^= 1u;
+                    }
+                };
+                if (!mbar_wait_bounded(&acc_empty[0], acc_phase ^ 1u, p.status, kDevTimeoutAcc)) break;
+                tc_fence_after();
+                int kb0 = kb_begin, ahead = 0, st = stage;
+                uint32_t ph = phase;
+                while (ok && ahead < STAGES && kb0 < kb_end && !mbar_try_wait(&acc_empty[1], acc_phase ^ 1u)) {
+                    ok = mbar_wait_bounded(&full[st], ph, p.status, kDevTimeoutFull);
+                    if (!ok) break;
+                    tc_fence_after();
+                    issue(st, kb0, true, false);
+                    kb0 += KPACK;
+                    ++ahead;
+                    next(st, ph);
                 }
+                if (ok) ok = mbar_wait_bounded(&acc_empty[1], acc_phase ^ 1u, p.status, kDevTimeoutAcc);
+                if (!ok) break;
                 acc_phase ^= 1u;
                 tc_fence_after();
-                const int kb_begin = (w % p.ksplit) * p.kb_split, kb_end = min(p.kblocks, kb_begin + p.kb_split);
-                for (int kb0 = kb_begin; kb0 < kb_end; kb0 += KPACK) {
+                for (int i = 0; i < ahead; ++i) {
+                    issue(stage, kb_begin + i * KPACK, false, true);
+                    tc_commit(&empty[stage]);  // frees the stage once these MMAs have read it
+                    next(stage, phase);
+                }
+                for (; kb0 < kb_end; kb0 += KPACK) {
                     if (!mbar_wait_bounded(&full[stage], phase, p.status, kDevTimeoutFull)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const int nkb = min(KPACK, kb_end - kb0);
-                    const uint32_t sa = smem_base + stage * STAGE_BYTES;
-                    const uint64_t a0 = sw32_desc(sa), b0 = sw32_desc(sa + KPACK * SLAB);
-#pragma unroll
-                    for (int j = 0; j < KPACK; ++j) {
-                        if (j < nkb) {
-                            const uint32_t acc = (kb0 + j > kb_begin) ? 1u : 0u;
-                            const uint64_t bj = b0 + (uint64_t)((j * SLAB) >> 4);
-                            tc_mma_i8(tmem_base, a0 + (uint64_t)((j * SLAB) >> 4), bj, IDESC_S8_128x256, acc);
-                            tc_mma_i8(tmem_base + 256, a0 + (uint64_t)((j * SLAB + SLAB / 2) >> 4), bj,
-                                      IDESC_S8_128x256, acc);
-                        }
+                    if (kb0 + KPACK < kb_end) {
+                        issue(stage, kb0, true, true);
+                    } else {  // accumulator 0 is done first, and drains while the other's MMAs run
+                        issue(stage, kb0, true, false);
+                        tc_commit(&acc_full[0]);
+                        issue(stage, kb0, false, true);
                     }
-                    tc_commit(&empty[stage]);  // frees the stage once these MMAs have read it
-                    if (++stage == STAGES) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
+                    tc_commit(&empty[stage]);
+                    next(stage, phase);
                 }
-                if (ok) tc_commit(acc_full);
+                if (ok) {
+                    if (kb_begin + ahead * KPACK >= kb_end) tc_commit(&acc_full[0]);  // all of it ran ahead
+                    tc_commit(&acc_full[1]);
+                }
             }
             // Drain: all MMAs this thread issued have finished before TMEM is released.
             tc_commit(drain);
@@ -715,31 +753,34 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
         }
     } else {
         // ------------------------------------------------------------ epilogue (warps 2..)
-        const int qd = warp & 3;            // TMEM lane quarter this warp may access
-        const int h = ((warp - 2) >> 2) & 1;  // accumulator: tile rows 0-127 or 128-255
-        const int c0 = ((warp - 2) >> 3) * EPI_CHUNKS;  // first 32-column chunk of this warp
+        const int qd = warp & 3;         // TMEM lane quarter this warp may access
+        const int c0 = (warp - 2) >> 2 << 1;  // first of its two 32-column chunks
         uint32_t acc_phase = 0;
-        for (int w = blockIdx.x; w < items; w += gridDim.x) {
-            bool got = true;
-            if (lane == 0) got = mbar_wait_sleepy(acc_full, acc_phase, p.status, kDevTimeoutAcc);
-            got = __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0;
-            if (!got) break;
-            acc_phase ^= 1u;
-            tc_fence_after();
+        bool ok = true;
+        for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
             int l, tm, tn, ks;
             item_of(p, w, l, tm, tn, ks);
             const uint32_t pm = (uint32_t)c_moduli[l], M = p.barrett[l], bias = p.bias[l];
             uint8_t *dst = p.rc + (size_t)ks * p.rc_slice + (size_t)l * p.rc_mod +
-                           ((size_t)tm * p.rc_tile_ld + tn) * OUT_TILE_BYTES +
-                           (size_t)((h * 4 + qd) * 32) * 256 + lane * 8;
-            const uint32_t tbase = tmem_base + ((uint32_t)(32 * qd) << 16) + h * 256;
-            // two 32-column loads in flight per wait, then their reduction and stores
+                           ((size_t)tm * p.rc_tile_ld + tn) * OUT_TILE_BYTES + (size_t)(qd * 32) * 256 + lane * 8;
 #pragma unroll 1
-            for (int c = c0; c < c0 + EPI_CHUNKS; c += 2) {
+            for (int h = 0; h < 2; ++h) {
+                bool got = true;
+                if (lane == 0) got = mbar_wait_sleepy(&acc_full[h], acc_phase, p.status, kDevTimeoutAcc);
+                got = __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0;
+                if (!got) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t tbase = tmem_base + ((uint32_t)(32 * qd) << 16) + h * 256;
                 uint32_t r[2][32];
-                tmem_ld32(tbase + c * 32, r[0]);
-                tmem_ld32(tbase + (c + 1) * 32, r[1]);
+                tmem_ld32(tbase + c0 * 32, r[0]);
+                tmem_ld32(tbase + (c0 + 1) * 32, r[1]);
                 tmem_wait_ld();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[h]);
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
                     uint32_t pk[8];
@@ -751,13 +792,11 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
                     }
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
-                        *reinterpret_cast<uint2 *>(dst + (size_t)(4 * (c + b) + u) * 256) =
+                        *reinterpret_cast<uint2 *>(dst + (size_t)h * (128 * 256) + (size_t)(4 * (c0 + b) + u) * 256) =
                             make_uint2(pk[2 * u], pk[2 * u + 1]);
                 }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty);
+            acc_phase ^= 1u;
         }
     }
 
