@@ -12,8 +12,9 @@
 //   h = 0; for d = s+1 down to 2: h = fma(h, 2^-7, G_d);   C_ij (+)= h * 2^(ea_i + eb_j - 12).
 //
 // Kernels:
-//   ozaki_row_exp   row maxima of A (one warp per row)
-//   ozaki_col_max   column maxima of B (atomicMax on the bit pattern of |b|)
+//   ozaki_row_exp   row maxima of A (one block per row); clears the column statistics
+//   ozaki_col_max   column maxima of B (atomicMax on the bit pattern of |b|); the last block of a
+//                   column group takes the exponents
 //   ozaki_split_a   digits of A as swizzled K-major tiles, blocked [row tile][K block][slice]
 //   ozaki_split_b   digits of B^T in the same layout, transposed through shared memory
 //   ozaki_gemm      persistent tcgen05 kernel, one 128 x 128 output tile at a time:
@@ -95,16 +96,51 @@ __device__ __forceinline__ double scale2(double x, int e)
 }
 
 // ---------------------------------------------------------------- split kernels
-__global__ void ozaki_row_exp(const double *__restrict__ A, int m, int k, int lda, int *__restrict__ ea,
-                              int *status)
+// What the column pass adds to and counts with, zeroed before it: by the row pass of the same split,
+// or by ozaki_zero.
+struct ColStats {
+    unsigned long long *max;  // per column
+    unsigned int *arrived;    // per group of 256 columns: blocks of ozaki_col_max that are done
+    int n;
+};
+
+__device__ __forceinline__ void zero_stats(const ColStats &z, long long i, long long step)
 {
-    const int warps = blockDim.x >> 5;
-    const int row = blockIdx.x * warps + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= m) return;
+    for (; i < z.n; i += step) {
+        z.max[i] = 0ull;
+        if (i % 256 == 0) z.arrived[i / 256] = 0u;
+    }
+}
+
+__global__ void __launch_bounds__(256) ozaki_zero(const ColStats z)
+{
+    pdl_wait();
+    pdl_trigger();
+    zero_stats(z, blockIdx.x * 256 + threadIdx.x, gridDim.x * 256ll);
+}
+
+// One block of T threads per row, eight loads in flight per thread (with one warp per row, a short, wide
+// A occupied a few SMs: the split phase of 128 x 2000 x 16384 took 318 us, 149 now).
+template <int T>
+__global__ void __launch_bounds__(T) ozaki_row_exp(const double *__restrict__ A, int m, int k, int lda,
+                                                   int *__restrict__ ea, const ColStats z, int *status)
+{
+    __shared__ unsigned long long red[T / 32];
+    pdl_wait();
+    pdl_trigger();
+    zero_stats(z, (long long)blockIdx.x * T + threadIdx.x, (long long)gridDim.x * T);
+    const int row = blockIdx.x;
     const unsigned long long *r = reinterpret_cast<const unsigned long long *>(A + (size_t)row * lda);
     unsigned long long mx = 0;
-    for (int kk = lane; kk < k; kk += 32) {
+    int kk = threadIdx.x;
+    for (; kk + 7 * T < k; kk += 8 * T) {
+        unsigned long long v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = __ldg(r + kk + u * T) & 0x7fffffffffffffffull;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) mx = v[u] > mx ? v[u] : mx;
+    }
+    for (; kk < k; kk += T) {
         const unsigned long long b = __ldg(r + kk) & 0x7fffffffffffffffull;
         mx = b > mx ? b : mx;
     }
@@ -112,7 +148,10 @@ __global__ void ozaki_row_exp(const double *__restrict__ A, int m, int k, int ld
         const unsigned long long other = __shfl_xor_sync(0xffffffffu, mx, o);
         mx = other > mx ? other : mx;
     }
-    if (lane == 0) {
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < T / 32; ++w) mx = red[w] > mx ? red[w] : mx;
         if (mx >= 0x7ff0000000000000ull) {
             ea[row] = NONFINITE_EXP;
             record_status(status, kDevNonFinite);
@@ -122,29 +161,42 @@ __global__ void ozaki_row_exp(const double *__restrict__ A, int m, int k, int ld
     }
 }
 
-// grid (ceil(n/256), ychunks); each thread scans a run of rows of one column.
-__global__ void ozaki_col_max(const double *__restrict__ B, int k, int n, int ldb, unsigned long long *colmax)
+// grid (ceil(n/256), ychunks); each thread scans a run of rows of one column, 8 loads in flight; the
+// last block of each column group to arrive takes the exponents.
+__global__ void __launch_bounds__(256) ozaki_col_max(const double *__restrict__ B, int k, int n, int ldb, const ColStats z,
+                                                     int *__restrict__ eb, int *status)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const int rows_per = (k + gridDim.y - 1) / gridDim.y;
-    const int r0 = blockIdx.y * rows_per;
-    const int r1 = min(k, r0 + rows_per);
-    unsigned long long mx = 0;
-    const unsigned long long *b = reinterpret_cast<const unsigned long long *>(B);
-    for (int r = r0; r < r1; ++r) {
-        const unsigned long long v = __ldg(b + (size_t)r * ldb + j) & 0x7fffffffffffffffull;
-        mx = v > mx ? v : mx;
+    __shared__ bool last;
+    pdl_wait();
+    pdl_trigger();
+    const int j = blockIdx.x * 256 + threadIdx.x;
+    if (j < n) {
+        const int rows_per = (k + gridDim.y - 1) / gridDim.y;
+        const int r0 = blockIdx.y * rows_per;
+        const int r1 = min(k, r0 + rows_per);
+        unsigned long long mx = 0;
+        const unsigned long long *b = reinterpret_cast<const unsigned long long *>(B) + j;
+        int r = r0;
+        for (; r + 8 <= r1; r += 8) {
+            unsigned long long v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = __ldg(b + (size_t)(r + u) * ldb) & 0x7fffffffffffffffull;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) mx = v[u] > mx ? v[u] : mx;
+        }
+        for (; r < r1; ++r) {
+            const unsigned long long v = __ldg(b + (size_t)r * ldb) & 0x7fffffffffffffffull;
+            mx = v > mx ? v : mx;
+        }
+        if (mx) atomicMax(z.max + j, mx);
     }
-    if (mx) atomicMax(colmax + j, mx);
-}
-
-__global__ void ozaki_col_exp(const unsigned long long *__restrict__ colmax, int n, int *__restrict__ eb,
-                              int *status)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const unsigned long long mx = colmax[j];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(z.arrived + blockIdx.x, 1u) == gridDim.y - 1;
+    __syncthreads();
+    if (!last || j >= n) return;
+    __threadfence();
+    const unsigned long long mx = __ldcg(z.max + j);
     if (mx >= 0x7ff0000000000000ull) {
         eb[j] = NONFINITE_EXP;
         record_status(status, kDevNonFinite);
@@ -153,26 +205,28 @@ __global__ void ozaki_col_exp(const unsigned long long *__restrict__ colmax, int
     }
 }
 
-// Digits of one value (the oracle's digits_of: d = rint(x), x <- (x - d) * 128).  rint is
-// computed by adding 1.5 * 2^52: for |x| < 2^51 the sum is rounded to an integer by the add
-// itself, to nearest with ties to even (as rint), and the integer sits in the low bits of the
-// sum.  Subtracting the constant back gives rint(x) exactly.  Two full-rate adds replace a
-// round and a float-to-int conversion per digit.
-template <int S>
-__device__ __forceinline__ void digits(double v, int e, int8_t (&d)[S], int s)
+// The S digits of eight values x = v 2^(6-e) (the oracle's digits_of: d = rint(x), x <- (x - d) * 128),
+// given to put(t, bytes) slice by slice, value j in byte j.  Digit t is the multiple of 2^(-7t) nearest
+// to what is left of x: adding 1.5 * 2^(52-7t) rounds to it (nearest, ties to even, as rint), leaves the
+// digit in the sum's low bits, and subtracting the constant and then the digit is exact.  Three FP64
+// additions per digit, two fewer for the last (x kept scaled by 128 took a fourth, and 64-bit shifts
+// to pack).  At 4096 x 4096 and 8 slices A's pass went from 54 to 46 us and B's from 82 to 42 (268 MB
+// each, 41 us at the measured HBM rate).
+template <int S, typename Put>
+__device__ __forceinline__ void digits8(double (&x)[8], const Put &put)
 {
-    constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52
-    double x = scale2(v, 6 - e);
 #pragma unroll
     for (int t = 0; t < S; ++t) {
-        if (t < s) {
-            const double y = __dadd_rn(x, kRound);
-            const double r = __dsub_rn(y, kRound);
-            d[t] = (int8_t)__double2loint(y);
-            x = (x - r) * 128.0;
-        } else {
-            d[t] = 0;
+        const double K = __longlong_as_double(__double_as_longlong(6755399441055744.0) - ((long long)(7 * t) << 52));
+        uint32_t d[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const double y = __dadd_rn(x[j], K);
+            d[j] = (uint32_t)__double2loint(y);
+            if (t + 1 < S) x[j] = __dsub_rn(x[j], __dsub_rn(y, K));
         }
+        put(t, make_uint2(__byte_perm(__byte_perm(d[0], d[1], 0x0040), __byte_perm(d[2], d[3], 0x0040), 0x5410),
+                          __byte_perm(__byte_perm(d[4], d[5], 0x0040), __byte_perm(d[6], d[7], 0x0040), 0x5410)));
     }
 }
 
@@ -186,79 +240,77 @@ __device__ __forceinline__ size_t slab_offset(int tile, int kb, int kblocks, int
     return ((size_t)tile * kblocks + kb) * (size_t)s * SLICE_TILE_BYTES + (size_t)r * 32 + (c ^ (((r >> 2) & 1) << 4));
 }
 
-// One warp per (8-row group, K block): lane -> row (lane / 4), 8 consecutive k (lane % 4).
+// Block: 64 rows of A x one 32-wide K block; warp w takes rows 8w..8w+7.  The rows are read whole
+// (32 consecutive doubles per load, whatever A's pitch) into a warp-private tile of 8 x 256 bytes
+// and handed on as lane -> row (lane / 4) and 8 consecutive k (lane % 4).  The 16-byte pieces of each
+// lane's 64 bytes are rotated so that the 16-byte reads are free of bank conflicts.
 // Rows up to the 128-row padding and k up to the 32 padding get zero digits.
 template <int S>
-__global__ void __launch_bounds__(256) ozaki_split_a(const double *__restrict__ A, int m, int k, int lda, int mp,
-                                                     int kblocks, const int *__restrict__ ea, uint8_t *__restrict__ da)
+__global__ void __launch_bounds__(256) ozaki_split_a(const double *__restrict__ A, int m, int k, int lda, int kblocks,
+                                                     const int *__restrict__ ea, uint8_t *__restrict__ da)
 {
-    const int lane = threadIdx.x & 31;
-    const long long wpb = blockDim.x >> 5;
-    const long long items = (long long)(mp / 8) * kblocks;
-    for (long long it = blockIdx.x * wpb + (threadIdx.x >> 5); it < items; it += (long long)gridDim.x * wpb) {
-        const int ro = (int)(it / kblocks), kb = (int)(it % kblocks);
-        const int row = ro * 8 + (lane >> 2), kq = lane & 3;
-        const int k0 = kb * 32 + kq * 8;
-        int e = (row < m) ? ea[row] : 0;
-        if (e == NONFINITE_EXP) e = 0;
-        unsigned long long packed[S];
+    __shared__ __align__(16) double tile[8][8][32];
+    pdl_wait();
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int kb = blockIdx.y, row0 = blockIdx.x * 64 + warp * 8, r = lane >> 2, kq = lane & 3, row = row0 + r;
+    {
+        const int kk = kb * 32 + lane;
+        const double *src = A + (size_t)row0 * lda + kk;
+        double v[8];
 #pragma unroll
-        for (int t = 0; t < S; ++t) packed[t] = 0;
-        const double *arow = A + (size_t)(row < m ? row : 0) * lda;
+        for (int i = 0; i < 8; ++i) v[i] = (row0 + i < m && kk < k) ? __ldg(src + (size_t)i * lda) : 0.0;
+        // 16-byte piece c = 4 q + j of row i goes to place 4 q + (j + q / 2 + 2 (i & 1)) % 4
+        const int q = lane >> 3, j = (lane >> 1) & 3;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int kk = k0 + j;
-            double v = (row < m && kk < k) ? __ldg(arow + kk) : 0.0;
-            if (!isfinite(v)) v = 0.0;
-            int8_t dg[S];
-            digits<S>(v, e, dg, S);
-#pragma unroll
-            for (int t = 0; t < S; ++t) packed[t] |= (unsigned long long)(uint8_t)dg[t] << (8 * j);
-        }
-        const size_t off = slab_offset(row >> 7, kb, kblocks, S, row & 127, kq * 8);
-#pragma unroll
-        for (int t = 0; t < S; ++t)
-            *reinterpret_cast<unsigned long long *>(da + off + (size_t)t * SLICE_TILE_BYTES) = packed[t];
+        for (int i = 0; i < 8; ++i)
+            tile[warp][i][(4 * q + ((j + (q >> 1) + 2 * (i & 1)) & 3)) * 2 + (lane & 1)] = v[i];
     }
+    int e = (row < m) ? ea[row] : 0;
+    const bool live = e != NONFINITE_EXP;  // a live row holds finite values only
+    if (!live) e = 0;
+    __syncwarp();
+    double x[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const double2 v = *reinterpret_cast<const double2 *>(&tile[warp][r][(4 * kq + ((j + (kq >> 1) + 2 * (r & 1)) & 3)) * 2]);
+        x[2 * j] = live ? scale2(v.x, 6 - e) : 0.0;
+        x[2 * j + 1] = live ? scale2(v.y, 6 - e) : 0.0;
+    }
+    uint8_t *dst = da + slab_offset(row >> 7, kb, kblocks, S, row & 127, kq * 8);
+    digits8<S>(x, [&](int t, uint2 b) { *reinterpret_cast<uint2 *>(dst + (size_t)t * SLICE_TILE_BYTES) = b; });
 }
 
-// Block: 32 k x 128 columns of B through shared memory (coalesced reads along the columns),
-// written as the digit tiles of B^T (column j of B is row j of the tile).
+// Block: 32 k x 64 columns of B through shared memory (coalesced reads along the columns), written as
+// the digit tiles of B^T (column j of B is row j of the tile): lane -> column (lane / 4) of the warp's
+// eight and 8 consecutive k (lane % 4).
 template <int S>
 __global__ void __launch_bounds__(256) ozaki_split_b(const double *__restrict__ B, int k, int n, int ldb, int kblocks,
                                                      const int *__restrict__ eb, uint8_t *__restrict__ db)
 {
-    __shared__ double tb[32][129];
-    const int tn = blockIdx.x, kb = blockIdx.y;
-    const int n0 = tn * 128, k0 = kb * 32;
-    for (int idx = threadIdx.x; idx < 32 * 128; idx += 256) {
-        const int kk = idx >> 7, c = idx & 127;
-        double v = (k0 + kk < k && n0 + c < n) ? __ldg(B + (size_t)(k0 + kk) * ldb + n0 + c) : 0.0;
-        if (!isfinite(v)) v = 0.0;
-        tb[kk][c] = v;
+    __shared__ double tb[32][65];
+    pdl_wait();
+    pdl_trigger();
+    const int n0 = blockIdx.x * 64, kb = blockIdx.y, k0 = kb * 32;
+    {
+        const int c = threadIdx.x & 63, kr = threadIdx.x >> 6;
+        const double *src = B + (size_t)(k0 + kr) * ldb + n0 + c;
+        double v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = (k0 + kr + 4 * i < k && n0 + c < n) ? __ldg(src + (size_t)(4 * i) * ldb) : 0.0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) tb[kr + 4 * i][c] = v[i];
     }
+    const int r = threadIdx.x >> 2, kq = threadIdx.x & 3, col = n0 + r;   // tile row r % 128 = column of B
+    int e = (col < n) ? eb[col] : 0;
+    const bool live = e != NONFINITE_EXP;  // a live column holds finite values only
+    if (!live) e = 0;
     __syncthreads();
+    double x[8];
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const int item = threadIdx.x + 256 * half;
-        const int r = item >> 2, kq = item & 3;   // tile row r = column n0 + r of B
-        int e = (n0 + r < n) ? eb[n0 + r] : 0;
-        if (e == NONFINITE_EXP) e = 0;
-        unsigned long long packed[S];
-#pragma unroll
-        for (int t = 0; t < S; ++t) packed[t] = 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            int8_t dg[S];
-            digits<S>(tb[kq * 8 + j][r], e, dg, S);
-#pragma unroll
-            for (int t = 0; t < S; ++t) packed[t] |= (unsigned long long)(uint8_t)dg[t] << (8 * j);
-        }
-        const size_t off = slab_offset(tn, kb, kblocks, S, r, kq * 8);
-#pragma unroll
-        for (int t = 0; t < S; ++t)
-            *reinterpret_cast<unsigned long long *>(db + off + (size_t)t * SLICE_TILE_BYTES) = packed[t];
-    }
+    for (int j = 0; j < 8; ++j) x[j] = live ? scale2(tb[kq * 8 + j][r], 6 - e) : 0.0;
+    uint8_t *dst = db + slab_offset(col >> 7, kb, kblocks, S, col & 127, kq * 8);
+    digits8<S>(x, [&](int t, uint2 b) { *reinterpret_cast<uint2 *>(dst + (size_t)t * SLICE_TILE_BYTES) = b; });
 }
 
 // ---------------------------------------------------------------- tcgen05 helpers
@@ -448,6 +500,8 @@ __global__ void __launch_bounds__(THREADS, 1) ozaki_gemm(const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();  // the set-up above overlaps the end of the previous kernel
+    pdl_trigger();
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
@@ -627,7 +681,7 @@ using namespace mgx;
 namespace {
 
 struct WsLayout {
-    size_t da, db, ea, eb, colmax, total;
+    size_t da, db, ea, eb, colmax, arrived, total;
     int kblocks;
 };
 
@@ -657,6 +711,8 @@ WsLayout ws_layout(int m, int n, int k, int s)
     off = align256(off + sizeof(int) * (size_t)n);
     L.colmax = off;
     off = align256(off + sizeof(unsigned long long) * (size_t)n);
+    L.arrived = off;   // per column group: blocks that are done with its maxima
+    off = align256(off + sizeof(unsigned int) * (size_t)((n + 255) / 256));
     L.total = off;
     return L;
 }
@@ -688,63 +744,74 @@ static int dispatch_splits(int s, Args... args)
 
 template <int S>
 struct SplitA {
-    static int run(const double *A, int m, int k, int lda, int mp, int kblocks, const int *ea, uint8_t *da,
-                   cudaStream_t stream)
+    static int run(const double *A, int m, int k, int lda, int kblocks, const int *ea, uint8_t *da, cudaStream_t stream)
     {
-        oz::ozaki_split_a<S><<<mgx_sm_count() * 16, 256, 0, stream>>>(A, m, k, lda, mp, kblocks, ea, da);
-        MGX_HOST_CHECK(cudaGetLastError());
+        MGX_HOST_CHECK(mgx_launch_dependent(oz::ozaki_split_a<S>, dim3((m + 127) / 128 * 2, kblocks), 256, 0, stream, A, m, k,
+                                            lda, kblocks, ea, da));
         return MGX_SUCCESS;
     }
 };
 
 template <int S>
 struct SplitB {
-    static int run(const double *B, int k, int n, int ldb, int np, int kblocks, const int *eb, uint8_t *db,
-                   cudaStream_t stream)
+    static int run(const double *B, int k, int n, int ldb, int kblocks, const int *eb, uint8_t *db, cudaStream_t stream)
     {
-        oz::ozaki_split_b<S><<<dim3(np / 128, kblocks), 256, 0, stream>>>(B, k, n, ldb, kblocks, eb, db);
-        MGX_HOST_CHECK(cudaGetLastError());
+        MGX_HOST_CHECK(mgx_launch_dependent(oz::ozaki_split_b<S>, dim3((n + 127) / 128 * 2, kblocks), 256, 0, stream, B, k, n,
+                                            ldb, kblocks, eb, db));
         return MGX_SUCCESS;
     }
 };
 
+static oz::ColStats col_stats(unsigned char *ws, const WsLayout &L, int n)
+{
+    oz::ColStats z;
+    z.max = reinterpret_cast<unsigned long long *>(ws + L.colmax);
+    z.arrived = reinterpret_cast<unsigned int *>(ws + L.arrived);
+    z.n = n;
+    return z;
+}
+
+// `zero`: column statistics for the row pass to clear.
 static int ozaki_split_a_impl(const double *A, int m, int k, int lda, int s, unsigned char *ws, const WsLayout &L,
-                              cudaStream_t stream)
+                              cudaStream_t stream, const oz::ColStats &zero = oz::ColStats{})
 {
     int *status = mgx_device_status_ptr();
     int *ea = reinterpret_cast<int *>(ws + L.ea);
     const int kblocks = (k + 31) / 32;
-    const int mp = (m + 127) / 128 * 128;
-    oz::ozaki_row_exp<<<(m + 7) / 8, 256, 0, stream>>>(A, m, k, lda, ea, status);
-    MGX_HOST_CHECK(cudaGetLastError());
-    return dispatch_splits<SplitA>(s, A, m, k, lda, mp, kblocks, (const int *)ea, ws + L.da, stream);
+    // enough threads that a row is a few batches of loads
+    auto scan = [&](auto kernel, int threads) {
+        return mgx_launch_dependent(kernel, dim3((unsigned)m), dim3(threads), 0, stream, A, m, k, lda, ea, zero, status);
+    };
+    MGX_HOST_CHECK(k <= 512    ? scan(oz::ozaki_row_exp<32>, 32)
+                   : k <= 2048 ? scan(oz::ozaki_row_exp<128>, 128)
+                               : scan(oz::ozaki_row_exp<256>, 256));
+    return dispatch_splits<SplitA>(s, A, m, k, lda, kblocks, (const int *)ea, ws + L.da, stream);
 }
 
+// `zeroed`: the column statistics are clear.
 static int ozaki_split_b_impl(const double *B, int n, int k, int ldb, int s, unsigned char *ws, const WsLayout &L,
-                              cudaStream_t stream)
+                              cudaStream_t stream, bool zeroed = false)
 {
     int *status = mgx_device_status_ptr();
     int *eb = reinterpret_cast<int *>(ws + L.eb);
-    unsigned long long *colmax = reinterpret_cast<unsigned long long *>(ws + L.colmax);
-    const int kblocks = (k + 31) / 32;
-    const int np = (n + 127) / 128 * 128;
+    const oz::ColStats z = col_stats(ws, L, n);
+    const int kblocks = (k + 31) / 32, groups = (n + 255) / 256;
     const int sms = mgx_sm_count();
-    MGX_HOST_CHECK(cudaMemsetAsync(colmax, 0, sizeof(unsigned long long) * (size_t)n, stream));
-    int ych = (sms * 8) / ((n + 255) / 256);
+    if (!zeroed)
+        MGX_HOST_CHECK(mgx_launch_dependent(oz::ozaki_zero, dim3((unsigned)(groups < 64 ? groups : 64)), 256, 0, stream, z));
+    int ych = (sms * 8) / groups;
     if (ych > (k + 63) / 64) ych = (k + 63) / 64;
     if (ych < 1) ych = 1;
-    oz::ozaki_col_max<<<dim3((n + 255) / 256, ych), 256, 0, stream>>>(B, k, n, ldb, colmax);
-    MGX_HOST_CHECK(cudaGetLastError());
-    oz::ozaki_col_exp<<<(n + 255) / 256, 256, 0, stream>>>(colmax, n, eb, status);
-    MGX_HOST_CHECK(cudaGetLastError());
-    return dispatch_splits<SplitB>(s, B, k, n, ldb, np, kblocks, (const int *)eb, ws + L.db, stream);
+    MGX_HOST_CHECK(mgx_launch_dependent(oz::ozaki_col_max, dim3((unsigned)groups, (unsigned)ych), 256, 0, stream, B, k, n, ldb,
+                                        z, eb, status));
+    return dispatch_splits<SplitB>(s, B, k, n, ldb, kblocks, (const int *)eb, ws + L.db, stream);
 }
 
 static int ozaki_split_impl(const double *A, const double *B, int m, int n, int k, int lda, int ldb, int s,
                             unsigned char *ws, const WsLayout &L, cudaStream_t stream)
 {
-    int rc = ozaki_split_a_impl(A, m, k, lda, s, ws, L, stream);
-    if (rc == MGX_SUCCESS) rc = ozaki_split_b_impl(B, n, k, ldb, s, ws, L, stream);
+    int rc = ozaki_split_a_impl(A, m, k, lda, s, ws, L, stream, col_stats(ws, L, n));
+    if (rc == MGX_SUCCESS) rc = ozaki_split_b_impl(B, n, k, ldb, s, ws, L, stream, true);
     return rc;
 }
 
@@ -831,17 +898,19 @@ static int ozaki_multiply_impl(double *C, int m, int n, int k, int ldc, int beta
         return MGX_E_WORKSPACE;
     }
     p.status = mgx_device_status_ptr();
-    p.sync = oz_sync_ptr(slot);
-    if (p.sync) MGX_HOST_CHECK(cudaMemsetAsync(p.sync, 0, sizeof(unsigned int), stream));
     const int smem = p.stages * p.stage_bytes + 1024 + 256;
     const int total = ((m + oz::TILE - 1) / oz::TILE) * ((n + oz::TILE - 1) / oz::TILE) * slices;
     const int sms = mgx_sm_count();
     const int grid = sms < total ? sms : total;
     if (grid < 1) return MGX_SUCCESS;
+    // the lockstep pays over many items; over few, clearing its counter costs more (as for the CRT form)
+    if (total >= 10ll * grid) {
+        p.sync = oz_sync_ptr(slot);
+        if (p.sync) MGX_HOST_CHECK(cudaMemsetAsync(p.sync, 0, sizeof(unsigned int), stream));
+    }
     auto launch = [&](auto kernel) -> int {
         MGX_HOST_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        kernel<<<grid, oz::THREADS, smem, stream>>>(p);
-        MGX_HOST_CHECK(cudaGetLastError());
+        MGX_HOST_CHECK(mgx_launch_dependent(kernel, dim3((unsigned)grid), dim3(oz::THREADS), smem, stream, p));
         if (slices > 1)  // C (+)= slice 0 + slice 1 + ..., in slice order
             return mgx_launch_splitk_reduce(C, ldc, beta_one, partial, p.partial_ld, p.partial_stride, slices, m, n,
                                             stream);
@@ -1067,6 +1136,8 @@ WsLayout ws_sub(const WsLayout &L, int r0, int c0, int s)
     S.ea = L.ea + sizeof(int) * (size_t)r0;
     S.eb = L.eb + sizeof(int) * (size_t)c0;
     S.colmax = L.colmax + sizeof(unsigned long long) * (size_t)c0;
+    // c0 is a multiple of 128: two panels may share a counter, but they follow each other on one stream
+    S.arrived = L.arrived + sizeof(unsigned int) * (size_t)(c0 / 256);
     return S;
 }
 
