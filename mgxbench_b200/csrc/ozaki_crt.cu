@@ -79,6 +79,13 @@ static_assert(STAGES >= 2 && STAGES <= 8, "pipeline depth");
 __constant__ int c_moduli[MAXQ] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
 static const int h_moduli[MAXQ] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
 
+// The same as compile-time constants: unrolled code takes them as immediates.
+__host__ __device__ constexpr uint32_t modulus(int l)
+{
+    constexpr uint32_t p[MAXQ] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
+    return p[l];
+}
+
 // Host-computed constants of one modulus set.
 struct Consts {
     int q, L, alpha, beta;
@@ -87,8 +94,6 @@ struct Consts {
     double w[MAXQ][3];     // CRT weights in 40-bit chunks, 2^974
     double pc[3];          // P in 40-bit chunks, 2^-60
     double inv_phat;       // 2^60 / (P / 2^(L-40))
-    double c32[MAXQ];      // 2^32 mod p_l
-    double inv_p[MAXQ];    // 1 / p_l (rounded)
     uint32_t barrett[MAXQ];  // ceil(2^32 / p_l)
 };
 
@@ -332,51 +337,109 @@ __global__ void __launch_bounds__(256) crt_col_sumsq(const double *__restrict__ 
 }
 
 // ---------------------------------------------------------------- residue kernels
-// Residues of one value: x = rint(v 2^sg) (|x| < 2^63) is split exactly into xh 2^32 + xl
-// (xl in [0, 2^32)); for each modulus y = xh (2^32 mod p) + xl (|y| < 2^40, exact) and
-// r = y - p rint(y / p), in [-(p-1)/2, (p-1)/2] for odd p, +-128 for 256.  A double
-// 1.5 * 2^52 + z with |z| < 2^51 an integer holds z mod 2^32 in its low word, so
-//   Y = fma(xh, c, xl + 1.5 * 2^52)   (exact)      -> low word y mod 2^32
-//   y = Y - 1.5 * 2^52                (exact)
-//   t = fma(y, 1/p, 1.5 * 2^52)       (one rounding) -> low word rint(y / p): y / p is never
-//       within 2^-9 of a half-integer for odd p, far above the error of the rounded 1/p
-// and r = lo(Y) - p lo(t) in 32-bit arithmetic (r is small, so the wrap-around cancels).
-// The kernels split 8 values first (split32) and then run each modulus over all 8
-// (residue_word): a modulus's constants are read once per 8 values, and the 8 residue bytes
-// pack into two words with byte permutes.
-constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52
+// Residues of one value: x = rint(v 2^sg) (|x| < 2^63) is split exactly into xh 2^32 + xl with
+// xh = rint(x 2^-32), |xl| <= 2^31, by adding 1.5 * 2^52: a double 1.5 * 2^52 + z with |z| < 2^51 is
+// rounded to an integer by the add itself (nearest, ties to even, as rint) and holds z mod 2^32
+// in its low word.  Two moduli p, p' share the FP64 part, their product pp <= 65280:
+//   Y = fma(xh, 2^32 mod pp, xl + 1.5 * 2^52)      exact; Y = 1.5 * 2^52 + y, |y| < 2^48, y = x (mod pp)
+//   t = fma(Y, 1/pp, magic)    low word off + rint(y / pp + d), |d| <= 1/2: the magic's rounding
+//   u = lo(Y) - pp lo(t)       the bits of the float M + z, z = x (mod pp), |z| <= pp + 4, where off
+//                              puts M's bits there (pp off = -bits(M) mod 2^32)
+// and each residue follows in FP32, r = z - p rint(z / p) in [-(p-1)/2, (p-1)/2] for odd p, +-128 for
+// 256, from q = fma(u, 1/p, 1.5 * 2^23 - rint(M/p)) and the low byte of u - p lo(q).  M in [2^23, 2^24)
+// is a multiple of 256 (so it does not touch the low byte) for which M (1/p) with the rounded 1/p
+// lies within 1.5 * 2^-10 of an integer for both moduli; z / p is never within 1 / (2p) of a
+// half-integer for odd p.  The pairs are those for which such an M exists.  tests/test_crt_residues.py
+// checks every z of every pair, and the first stage against exact integers.
+// Bound by issue slots: 3.5 instructions per residue, one of them FP64 (two slots of that pipe), and
+// 0.75 to pack the bytes.  With three FP64 operations and an integer one per modulus, rint and floor
+// conversions and a finiteness test per value, it was 119 instructions per value.  SPLITFIG
+// The kernels split 8 values first (split32) and then run each pair over all 8 (all_residues).
+constexpr double kRound = 6755399441055744.0;            // 1.5 * 2^52
+constexpr double kRoundF = 12582912.0;                   // 1.5 * 2^23
 
-// x = rint(v 2^sg) as xh 2^32 + xl; returns xh and xl + 1.5 * 2^52.
+struct ModulusPair {
+    int a, b, M;   // indices of the moduli
+};
+struct PairSet {
+    ModulusPair pair[MAXQ / 2];
+    int single;    // the modulus left over where q is odd, else -1
+};
+constexpr PairSet kPairs[MAXQ - MINQ + 1] = {
+    /*  8 */ {{{0, 3, 8481792}, {1, 5, 14687744}, {2, 6, 15112448}, {4, 7, 14733056}}, -1},
+    /*  9 */ {{{0, 2, 16666880}, {1, 5, 14687744}, {4, 8, 14480128}, {6, 7, 14255872}}, 3},
+    /* 10 */ {{{0, 3, 8481792}, {1, 5, 14687744}, {2, 6, 15112448}, {4, 9, 13784576}, {7, 8, 13659392}}, -1},
+    /* 11 */ {{{0, 3, 8481792}, {1, 5, 14687744}, {2, 6, 15112448}, {4, 8, 14480128}, {7, 10, 14792704}}, 9},
+    /* 12 */ {{{0, 9, 16690176}, {1, 5, 14687744}, {2, 4, 15112448}, {3, 10, 13879296}, {6, 7, 14255872}, {8, 11, 12721408}}, -1},
+    /* 13 */ {{{0, 3, 8481792}, {1, 5, 14687744}, {2, 12, 16602112}, {4, 11, 13721344}, {6, 8, 14011136}, {7, 10, 14792704}}, 9},
+    /* 14 */ {{{0, 9, 16690176}, {1, 5, 14687744}, {2, 12, 16602112}, {3, 13, 12786944}, {4, 8, 14480128}, {6, 11, 13276928}, {7, 10, 14792704}}, -1},
+    /* 15 */ {{{0, 3, 8481792}, {1, 5, 14687744}, {2, 12, 16602112}, {4, 11, 13721344}, {6, 7, 14255872}, {8, 13, 11666176}, {10, 14, 14221824}}, 9},
+    /* 16 */ {{{0, 9, 16690176}, {1, 5, 14687744}, {2, 12, 16602112}, {3, 15, 12401408}, {4, 7, 14733056}, {6, 8, 14011136}, {10, 14, 14221824}, {11, 13, 11054848}}, -1}};
+
+// off with pp off = -bits(M) (mod 2^32); bits(M) is a multiple of 256, which covers an even pp.
+constexpr uint32_t pair_offset(uint32_t pp, int M)
+{
+    const uint32_t bits = 0x4B000000u + (uint32_t)(M - (1 << 23));
+    const bool even = pp % 2 == 0;
+    const uint32_t odd = even ? pp / 256 : pp, target = 0u - (even ? bits / 256 : bits);
+    uint32_t inv = odd;  // Newton's iteration for odd^-1 mod 2^32
+    for (int i = 0; i < 5; ++i) inv *= 2u - odd * inv;
+    return target * inv & (even ? 0xffffffu : 0xffffffffu);
+}
+
+// x = rint(v 2^sg) as xh 2^32 + xl; returns xh and xl + kRound.
 __device__ __forceinline__ void split32(double v, double f1, double f2, double &xh, double &xr)
 {
-    const double x = rint(__dmul_rn(__dmul_rn(v, f1), f2));
-    xh = floor(__dmul_rn(x, 2.3283064365386963e-10));  // x * 2^-32
+    const double x = __dmul_rn(__dmul_rn(v, f1), f2);
+    xh = __dsub_rn(__fma_rn(x, 2.3283064365386963e-10, kRound), kRound);  // rint(x * 2^-32)
     xr = __dadd_rn(__fma_rn(-xh, 4294967296.0, x), kRound);
 }
 
-// The residue mod p as the low byte of the returned word (c = 2^32 mod p, ip = 1/p).
-__device__ __forceinline__ uint32_t residue_word(double xh, double xr, double c, double ip, uint32_t p)
+// Low bytes of w[0..7], w[0] in the lowest byte.
+__device__ __forceinline__ uint2 pack8(const uint32_t (&w)[8])
 {
-    const double Y = __fma_rn(xh, c, xr);
-    const double t = __fma_rn(__dsub_rn(Y, kRound), ip, kRound);
-    return (uint32_t)__double2loint(Y) - (uint32_t)__double2loint(t) * p;
-}
-
-// Low bytes of a, b, c, d as one word (a in the lowest byte).
-__device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, uint32_t d)
-{
-    return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
-}
-
-// The 8 residue bytes of xh/xr[0..7] for modulus l, element j in byte j.
-__device__ __forceinline__ uint2 residues8(const double (&xh)[8], const double (&xr)[8], const Consts &K, int l)
-{
-    const double c = K.c32[l], ip = K.inv_p[l];
-    const uint32_t p = (uint32_t)c_moduli[l];
-    uint32_t w[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) w[j] = residue_word(xh[j], xr[j], c, ip, p);
+    auto pack4 = [](uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+        return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+    };
     return make_uint2(pack4(w[0], w[1], w[2], w[3]), pack4(w[4], w[5], w[6], w[7]));
+}
+
+// All Q moduli's residue bytes of xh/xr[0..7], element j in byte j, given to put(l, bytes).
+template <int Q, int I = 0, typename Put>
+__device__ __forceinline__ void all_residues(const double (&xh)[8], const double (&xr)[8], const Put &put)
+{
+    constexpr PairSet set = kPairs[Q - MINQ];
+    uint32_t w0[8], w1[8];
+    if constexpr (I < Q / 2) {
+        constexpr int a = set.pair[I].a, b = set.pair[I].b, M = set.pair[I].M;
+        constexpr uint32_t p0 = modulus(a), p1 = modulus(b), pp = p0 * p1;
+        constexpr double c = (double)((1ull << 32) % pp), ip = 1.0 / (double)pp;
+        constexpr double magic = kRound + (double)pair_offset(pp, M) - (double)(long long)(kRound * ip + 0.5);
+        constexpr float ip0 = 1.0f / (float)p0, ip1 = 1.0f / (float)p1;
+        constexpr float c0 = (float)(kRoundF - (double)(long long)((double)M * (double)ip0 + 0.5));
+        constexpr float c1 = (float)(kRoundF - (double)(long long)((double)M * (double)ip1 + 0.5));
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const double Y = __fma_rn(xh[j], c, xr[j]);
+            const double t = __fma_rn(Y, ip, magic);
+            const uint32_t u = (uint32_t)__double2loint(Y) + (uint32_t)__double2loint(t) * (0u - pp);
+            w0[j] = u + __float_as_uint(__fmaf_rn(__uint_as_float(u), ip0, c0)) * (0u - p0);
+            w1[j] = u + __float_as_uint(__fmaf_rn(__uint_as_float(u), ip1, c1)) * (0u - p1);
+        }
+        put(a, pack8(w0));
+        put(b, pack8(w1));
+        all_residues<Q, I + 1>(xh, xr, put);
+    } else if constexpr (set.single >= 0) {
+        constexpr uint32_t p0 = modulus(set.single);
+        constexpr double c = (double)((1ull << 32) % p0), ip = 1.0 / (double)p0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const double Y = __fma_rn(xh[j], c, xr[j]);
+            const double t = __fma_rn(__dsub_rn(Y, kRound), ip, kRound);  // rint(y / p): the residue is exact
+            w0[j] = (uint32_t)__double2loint(Y) + (uint32_t)__double2loint(t) * (0u - p0);
+        }
+        put(set.single, pack8(w0));
+    }
 }
 
 // Slab layout: byte (row r, k byte c) of K block kb of 256-row tile t of modulus l sits at
@@ -387,39 +450,48 @@ __device__ __forceinline__ size_t slab_offset(int tile, int kb, int kblocks, int
     return ((size_t)tile * kblocks + kb) * (size_t)SLAB + (size_t)r * 32 + (c ^ (((r >> 2) & 1) << 4));
 }
 
-// Block: 64 rows of A x one 32-wide K block; warp w takes rows 8w..8w+7, lane -> row (lane / 4)
-// and 8 consecutive k (lane % 4), so four lanes read one 256-byte row segment and write the 32
-// residue bytes of that row, one 8-byte store each per modulus.
+// Block: 64 rows of A x one 32-wide K block; warp w takes rows 8w..8w+7.  The rows are read whole
+// (32 consecutive doubles per load, whatever A's pitch) into a warp-private tile of 8 x 256 bytes
+// and handed on as lane -> row (lane / 4) and 8 consecutive k (lane % 4), so four lanes write the 32
+// residue bytes of a row, one 8-byte store each per modulus.  The 16-byte pieces of each lane's
+// 64 bytes are rotated so that the 16-byte reads are free of bank conflicts.
 template <int Q>
-__global__ void __launch_bounds__(256, 3) crt_split_a(const double *__restrict__ A, int m, int k, int lda, int mp,
-                                                      int kblocks, const int *__restrict__ sg, uint8_t *__restrict__ ra,
-                                                      size_t mod_stride, const __grid_constant__ Consts K)
+__global__ void __launch_bounds__(256, 4) crt_split_a(const double *__restrict__ A, int m, int k, int lda, int kblocks,
+                                                      const int *__restrict__ sg, uint8_t *__restrict__ ra,
+                                                      size_t mod_stride)
 {
+    __shared__ __align__(16) double tile[8][8][32];
     pdl_wait();
     pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int kb = blockIdx.y;
-    const int row = blockIdx.x * 64 + warp * 8 + (lane >> 2), kq = lane & 3;
-    if (row >= mp) return;
-    const int k0 = kb * 32 + kq * 8;
+    const int kb = blockIdx.y, row0 = blockIdx.x * 64 + warp * 8, r = lane >> 2, kq = lane & 3, row = row0 + r;
+    {
+        const int kk = kb * 32 + lane;
+        const double *src = A + (size_t)row0 * lda + kk;
+        double v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = (row0 + i < m && kk < k) ? __ldg(src + (size_t)i * lda) : 0.0;
+        // 16-byte piece c = 4 q + j of row i goes to place 4 q + (j + q / 2 + 2 (i & 1)) % 4
+        const int q = lane >> 3, j = (lane >> 1) & 3;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            tile[warp][i][(4 * q + ((j + (q >> 1) + 2 * (i & 1)) & 3)) * 2 + (lane & 1)] = v[i];
+    }
+    // the residues of a row that is not finite do not matter: its results are NaN
     int s = (row < m) ? sg[row] : 0;
-    const bool live = row < m && s != NONFINITE;
-    if (!live) s = 0;
+    if (s == NONFINITE) s = 0;
     double f1, f2;
     scale_factors(s, f1, f2);
-    const double *arow = A + (size_t)(live ? row : 0) * lda;
+    __syncwarp();
     double xh[8], xr[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int kk = k0 + j;
-        double v = (live && kk < k) ? __ldg(arow + kk) : 0.0;
-        if (!isfinite(v)) v = 0.0;
-        split32(v, f1, f2, xh[j], xr[j]);
+    for (int j = 0; j < 4; ++j) {
+        const double2 v = *reinterpret_cast<const double2 *>(&tile[warp][r][(4 * kq + ((j + (kq >> 1) + 2 * (r & 1)) & 3)) * 2]);
+        split32(v.x, f1, f2, xh[2 * j], xr[2 * j]);
+        split32(v.y, f1, f2, xh[2 * j + 1], xr[2 * j + 1]);
     }
-    const size_t off = slab_offset(row / TILE, kb, kblocks, row % TILE, kq * 8);
-#pragma unroll
-    for (int l = 0; l < Q; ++l)
-        *reinterpret_cast<uint2 *>(ra + (size_t)l * mod_stride + off) = residues8(xh, xr, K, l);
+    uint8_t *dst = ra + slab_offset(row / TILE, kb, kblocks, row % TILE, kq * 8);
+    all_residues<Q>(xh, xr, [&](int l, uint2 b) { *reinterpret_cast<uint2 *>(dst + (size_t)l * mod_stride) = b; });
 }
 
 // Block: 64 consecutive columns of B x one 32-wide K block.  Warp w takes 32 of the columns
@@ -429,9 +501,9 @@ __global__ void __launch_bounds__(256, 3) crt_split_a(const double *__restrict__
 // one contiguous 2 KiB run of the slab (column j of B is row j % 256 of slab tile j / 256),
 // written out with 16-byte stores.
 template <int Q>
-__global__ void __launch_bounds__(256, 3) crt_split_b(const double *__restrict__ B, int k, int n, int ldb, int kblocks,
+__global__ void __launch_bounds__(256, 4) crt_split_b(const double *__restrict__ B, int k, int n, int ldb, int kblocks,
                                                       const int *__restrict__ tu, uint8_t *__restrict__ rb,
-                                                      size_t mod_stride, const __grid_constant__ Consts K)
+                                                      size_t mod_stride)
 {
     __shared__ __align__(16) unsigned char st[Q][64 * 32];
     pdl_wait();
@@ -441,22 +513,19 @@ __global__ void __launch_bounds__(256, 3) crt_split_b(const double *__restrict__
     const int rl = (warp >> 2) * 32 + lane;          // row of the block's 64
     const int col = blockIdx.x * 64 + rl;
     int s = (col < n) ? tu[col] : 0;
-    const bool live = col < n && s != NONFINITE;
-    if (!live) s = 0;
-    const double *bcol = B + (live ? col : 0);
+    if (s == NONFINITE) s = 0;   // as for A's rows
+    const double *bcol = B + (col < n ? col : 0);
     double f1, f2;
     scale_factors(s, f1, f2);
     double xh[8], xr[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const int kk = kb * 32 + kq * 8 + j;
-        double v = (live && kk < k) ? __ldg(bcol + (size_t)kk * ldb) : 0.0;
-        if (!isfinite(v)) v = 0.0;
+        const double v = (col < n && kk < k) ? __ldg(bcol + (size_t)kk * ldb) : 0.0;
         split32(v, f1, f2, xh[j], xr[j]);
     }
     const int soff = rl * 32 + ((kq * 8) ^ (((rl >> 2) & 1) << 4));
-#pragma unroll
-    for (int l = 0; l < Q; ++l) *reinterpret_cast<uint2 *>(&st[l][soff]) = residues8(xh, xr, K, l);
+    all_residues<Q>(xh, xr, [&](int l, uint2 b) { *reinterpret_cast<uint2 *>(&st[l][soff]) = b; });
     __syncthreads();
     const int c0 = blockIdx.x * 64;
     unsigned char *dst = rb + ((size_t)(c0 / TILE) * kblocks + kb) * (size_t)SLAB + (size_t)(c0 % TILE) * 32;
@@ -1016,8 +1085,6 @@ static bool make_consts(int q, Consts &K)
         while ((mm * inv) % p != 1) ++inv;
         chunks40(M * inv, L, K.w[l]);
         for (double &c : K.w[l]) c = ldexp(c, 1034 - kCombineShift);
-        K.c32[l] = (double)((1ull << 32) % p);
-        K.inv_p[l] = 1.0 / (double)p;
         K.barrett[l] = (uint32_t)(0xffffffffull / p + 1);
     }
     chunks40(P, L, K.pc);
@@ -1106,11 +1173,11 @@ int dispatch_q(int q, Args... args)
 template <int Q>
 struct SplitA {
     static int run(const double *A, int m, int k, int lda, const CrtLayout &L, const int *sg, uint8_t *ra,
-                   const crt::Consts &K, cudaStream_t stream)
+                   cudaStream_t stream)
     {
         const int tiles = (m + crt::TILE - 1) / crt::TILE;
         MGX_HOST_CHECK(mgx_launch_dependent(crt::crt_split_a<Q>, dim3(tiles * 4, L.kblocks), 256, 0, stream, A, m, k, lda,
-                                            tiles * crt::TILE, L.kblocks, sg, ra, L.ra_mod, K));
+                                            L.kblocks, sg, ra, L.ra_mod));
         return MGX_SUCCESS;
     }
 };
@@ -1118,11 +1185,11 @@ struct SplitA {
 template <int Q>
 struct SplitB {
     static int run(const double *B, int n, int k, int ldb, const CrtLayout &L, const int *tu, uint8_t *rb,
-                   const crt::Consts &K, cudaStream_t stream)
+                   cudaStream_t stream)
     {
         const int tiles = (n + crt::TILE - 1) / crt::TILE;
         MGX_HOST_CHECK(mgx_launch_dependent(crt::crt_split_b<Q>, dim3(tiles * 4, L.kblocks), 256, 0, stream, B, k, n, ldb,
-                                            L.kblocks, tu, rb, L.rb_mod, K));
+                                            L.kblocks, tu, rb, L.rb_mod));
         return MGX_SUCCESS;
     }
 };
@@ -1166,7 +1233,7 @@ int crt_split_a_impl(const double *A, int m, int k, int lda, int r0, const crt::
                    : k <= 4096 ? scale(crt::crt_row_scale<256, 16>, 256)
                    : k <= 8192 ? scale(crt::crt_row_scale<512, 16>, 512)
                                : scale(crt::crt_row_scale<512, 0>, 512));
-    return dispatch_q<SplitA>(K.q, A, m, k, lda, L, (const int *)sg, ra, K, stream);
+    return dispatch_q<SplitA>(K.q, A, m, k, lda, L, (const int *)sg, ra, stream);
 }
 
 // The same for columns [c0, c0 + n) of B (k x n).  `zeroed`: their statistics are clear.
@@ -1188,7 +1255,7 @@ int crt_split_b_impl(const double *B, int n, int k, int ldb, int c0, const crt::
     const dim3 grid((unsigned)groups, (unsigned)ych);
     MGX_HOST_CHECK(mgx_launch_dependent(crt::crt_col_max, grid, 256, 0, stream, B, k, n, ldb, z.max));
     MGX_HOST_CHECK(mgx_launch_dependent(crt::crt_col_sumsq, grid, 256, 0, stream, B, k, n, ldb, z, K.beta, tu, status));
-    return dispatch_q<SplitB>(K.q, B, n, k, ldb, L, (const int *)tu, rb, K, stream);
+    return dispatch_q<SplitB>(K.q, B, n, k, ldb, L, (const int *)tu, rb, stream);
 }
 
 int crt_split_impl(const double *A, const double *B, int m, int n, int k, int lda, int ldb, const crt::Consts &K,
