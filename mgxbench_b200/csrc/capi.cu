@@ -44,7 +44,7 @@ static int current_device()
 // Id of the context current on this thread (cuCtxGetId), 0 when there is none yet or the driver
 // lacks the call.  A context that cudaDeviceReset ended and the runtime later re-created gets a
 // new id, so an address cached under the old id is known to be stale.
-static unsigned long long current_context_id()
+unsigned long long mgx_context_id()
 {
     static PFN_cuCtxGetCurrent_v4000 get_current = nullptr;
     static PFN_cuCtxGetId_v12000 get_id = nullptr;
@@ -90,7 +90,7 @@ void *mgx_symbol_address(const void *symbol, int slot, cudaError_t *err)
     }
     std::lock_guard<std::mutex> lk(g_mu);
     Entry &e = cache[slot][dev];
-    unsigned long long ctx = current_context_id();
+    unsigned long long ctx = mgx_context_id();
     if (e.ptr && ctx != 0 && ctx == e.ctx) return e.ptr;
     void *p = nullptr;
     const cudaError_t rc = cudaGetSymbolAddress(&p, symbol);
@@ -101,7 +101,7 @@ void *mgx_symbol_address(const void *symbol, int slot, cudaError_t *err)
         return nullptr;
     }
     // The lookup itself creates the primary context when none was current yet.
-    if (ctx == 0) ctx = current_context_id();
+    if (ctx == 0) ctx = mgx_context_id();
     e.ctx = ctx;
     e.ptr = p;
     return p;

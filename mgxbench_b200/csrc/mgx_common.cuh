@@ -28,6 +28,7 @@ int *mgx_device_status_ptr();  // device address of this device's status word (n
 enum MgxSymbolSlot : int { kMgxSymStatus = 0, kMgxSymOzSync = 1, kMgxSymOzakiNoalloc = 2, kMgxSymbolSlots = 3 };
 void *mgx_symbol_address(const void *symbol, int slot, cudaError_t *err = nullptr);
 int mgx_sm_count();
+unsigned long long mgx_context_id();  // id of the context current on this thread, 0 if none
 // Stream-ordered scratch from the library's pool on the current device (free with cudaFreeAsync).
 int mgx_scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream);
 int mgx_encode_tmap_2d(CUtensorMap *map, CUtensorMapDataType dtype, int elem_bytes, const void *base,

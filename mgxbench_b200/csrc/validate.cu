@@ -25,9 +25,10 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long *addr, doub
     if (v > 0.0) atomicMax(addr, (unsigned long long)__double_as_longlong(v));
 }
 
-struct ConstAcc {
+// What one block of the constant check found.
+struct ConstPart {
     unsigned long long invalid;
-    unsigned long long max_abs_bits;
+    double max_abs;
 };
 
 // Bound by reading C from HBM: two 16-byte loads in flight per thread and no division.  The relative
@@ -37,7 +38,7 @@ struct ConstAcc {
 // 357 us with a division per element and one 8-byte load in flight, 94 us now (5.7 TB/s).
 __global__ void __launch_bounds__(THREADS) validate_const_kernel(const double *__restrict__ C, size_t count,
                                                                  double expected, double abs_tol, double rel_tol,
-                                                                 ConstAcc *acc)
+                                                                 ConstPart *parts)
 {
     unsigned long long bad = 0;
     double mabs = 0.0;
@@ -91,8 +92,7 @@ __global__ void __launch_bounds__(THREADS) validate_const_kernel(const double *_
             bad += s_bad[k];
             mabs = fmax(mabs, s_abs[k]);
         }
-        if (bad) atomicAdd(&acc->invalid, bad);
-        atomic_max_nonneg(&acc->max_abs_bits, mabs);
+        parts[blockIdx.x] = ConstPart{bad, mabs};
     }
 }
 
@@ -216,36 +216,81 @@ static double bits_to_double(unsigned long long b)
     return d;
 }
 
+namespace {
+
+// Page-locked memory the constant check's blocks write their findings to and the calling thread reads:
+// 32 KiB per host thread and device, given back when the thread ends, taken anew when the device's
+// context has changed since (a cudaDeviceReset freed it then).  With device accumulators, the call had
+// an allocation, a memset, a copy back through pageable memory and a free around its kernel.
+constexpr int kParts = 2048, kDevices = 64;
+
+struct PartsBuffers {
+    struct Slot {
+        val::ConstPart *ptr;
+        unsigned long long ctx;
+    } slot[kDevices] = {};
+
+    ~PartsBuffers()
+    {
+        int current = -1;
+        if (cudaGetDevice(&current) != cudaSuccess) return;
+        for (int d = 0; d < kDevices; ++d)
+            if (slot[d].ptr && cudaSetDevice(d) == cudaSuccess) {
+                if (mgx_context_id() == slot[d].ctx) cudaFreeHost(slot[d].ptr);
+                cudaSetDevice(current);
+            }
+    }
+
+    int take(val::ConstPart **out)
+    {
+        int d = 0;
+        MGX_HOST_CHECK(cudaGetDevice(&d));
+        if (d >= kDevices) {
+            mgx_set_last_message("constant validation: device %d is beyond %d", d, kDevices);
+            return MGX_E_UNSUPPORTED;
+        }
+        Slot &s = slot[d];
+        if (!s.ptr || mgx_context_id() != s.ctx) {
+            s.ptr = nullptr;
+            MGX_HOST_CHECK(cudaHostAlloc(reinterpret_cast<void **>(&s.ptr), kParts * sizeof(val::ConstPart),
+                                         cudaHostAllocPortable | cudaHostAllocMapped));
+            s.ctx = mgx_context_id();
+        }
+        *out = s.ptr;
+        return MGX_SUCCESS;
+    }
+};
+
+}  // namespace
+
 int mgx_validate_impl(const double *d_c, size_t count, double expected, double abs_tol, double rel_tol,
                       mgx_validation_t *out, cudaStream_t stream)
 {
-    val::ConstAcc h{0, 0};
+    out->elements = count;
+    out->invalid = 0;
+    out->max_abs_error = out->max_rel_error = 0.0;
     if (count > 0) {
-        val::ConstAcc *d_acc = nullptr;
-        {
-            const int arc = mgx_scratch_alloc(reinterpret_cast<void **>(&d_acc), sizeof(val::ConstAcc), stream);
-            if (arc != MGX_SUCCESS) return arc;
-        }
-        cudaError_t e = cudaMemsetAsync(d_acc, 0, sizeof(val::ConstAcc), stream);
-        if (e == cudaSuccess) {
-            size_t blocks = (count + 4 * val::THREADS - 1) / (4 * val::THREADS);  // four elements per step
-            const size_t cap = (size_t)mgx_sm_count() * 8;
-            if (blocks > cap) blocks = cap;
-            val::validate_const_kernel<<<(unsigned)blocks, val::THREADS, 0, stream>>>(d_c, count, expected, abs_tol,
-                                                                                      rel_tol, d_acc);
-            e = cudaGetLastError();
-        }
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d_acc, sizeof h, cudaMemcpyDeviceToHost, stream);
-        cudaFreeAsync(d_acc, stream);
+        static thread_local PartsBuffers buffers;
+        val::ConstPart *parts = nullptr;
+        const int brc = buffers.take(&parts);
+        if (brc != MGX_SUCCESS) return brc;
+        size_t blocks = (count + 4 * val::THREADS - 1) / (4 * val::THREADS);  // four elements per step
+        const size_t cap = (size_t)mgx_sm_count() * 8;
+        if (blocks > cap) blocks = cap;
+        if (blocks > kParts) blocks = kParts;
+        val::validate_const_kernel<<<(unsigned)blocks, val::THREADS, 0, stream>>>(d_c, count, expected, abs_tol, rel_tol,
+                                                                                  parts);
+        cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) {
             mgx_set_last_cuda_error(e, "constant validation", __FILE__, __LINE__);
             return MGX_E_CUDA;
         }
+        for (size_t b = 0; b < blocks; ++b) {
+            out->invalid += parts[b].invalid;
+            if (parts[b].max_abs > out->max_abs_error) out->max_abs_error = parts[b].max_abs;
+        }
     }
-    out->elements = count;
-    out->invalid = h.invalid;
-    out->max_abs_error = bits_to_double(h.max_abs_bits);
     // an infinite `expected` gives NaN quotients, which never count
     const double rel = fabs(expected) > 0.0 ? out->max_abs_error / fabs(expected) : 0.0;
     out->max_rel_error = rel > 0.0 ? rel : 0.0;

@@ -30,3 +30,28 @@ def test_limit_values_match_the_oracle(mgx, oracle, expected):
         n, ma, mr = oracle.validate_constant(C, expected, count_nonfinite=True)
     ok, v = mgx.validate_matrix_c(dev(C), 1, C.size, expected)
     assert v.invalid == n and v.max_abs_error == ma and v.max_rel_error == mr and ok == (n == 0)
+
+
+def test_threads_and_streams_check_at_the_same_time(mgx):
+    """Each host thread reads its own findings, whatever the others check meanwhile."""
+    import threading
+    import torch
+    xs = [torch.full((300 + 40 * i, 700), 8.0, dtype=torch.float64, device="cuda") for i in range(6)]
+    for i, x in enumerate(xs):
+        x[i, :i + 1] = 9.0 + i
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        for _ in range(20):
+            ok, v = mgx.validate_matrix_c(xs[i], xs[i].shape[0], 700, 8.0)
+            if ok or v.invalid != i + 1 or v.max_abs_error != 1.0 + i or v.max_rel_error != (1.0 + i) / 8.0:
+                bad.append((i, v.invalid, v.max_abs_error))
+
+    for _ in range(2):      # the second round's threads start after the first round's have ended
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(6)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    assert not bad
