@@ -40,21 +40,32 @@ int mgx_encode_tmap_3d(CUtensorMap *map, CUtensorMapDataType dtype, int elem_byt
 
 // Programmatic dependent launch: the kernel may be scheduled while the one before it in the stream
 // drains.  It must execute pdl_wait() before it touches memory; pdl_trigger() lets the next one in.
+// cluster > 1: thread-block clusters of that many CTAs along x.
 template <typename... Params, typename... Args>
-static inline cudaError_t mgx_launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
-                                               cudaStream_t stream, const Args &...args)
+static inline cudaError_t mgx_launch_dependent_cluster(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                                                       cudaStream_t stream, int cluster, const Args &...args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+template <typename... Params, typename... Args>
+static inline cudaError_t mgx_launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                                               cudaStream_t stream, const Args &...args)
+{
+    return mgx_launch_dependent_cluster(kernel, grid, block, smem, stream, 1, args...);
 }
 
 namespace mgx {
@@ -189,16 +200,6 @@ __device__ __forceinline__ void tma_load_2d(void *smem_dst, const CUtensorMap *m
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
             smem_u32(smem_dst)),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-        : "memory");
-}
-
-__device__ __forceinline__ void tma_load_3d(void *smem_dst, const CUtensorMap *map, int c0, int c1, int c2,
-                                            uint64_t *bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::
-            "r"(smem_u32(smem_dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
         : "memory");
 }
 

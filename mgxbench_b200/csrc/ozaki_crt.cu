@@ -46,13 +46,6 @@
 
 #include "mgx_common.cuh"
 
-#ifndef MGX_CRT_KPACK
-#define MGX_CRT_KPACK 4
-#endif
-#ifndef MGX_CRT_LOCKSTEP
-#define MGX_CRT_LOCKSTEP 1
-#endif
-
 namespace mgx {
 namespace crt {
 
@@ -62,19 +55,14 @@ constexpr int KMAX = 130816;           // 4088 K blocks: k * 128 * 128 < 2^31
 constexpr int TILE = 256;              // output tile TILE x TILE, operand slabs TILE rows
 constexpr int KB = 32;                 // bytes of K per MMA
 constexpr int SLAB = TILE * KB;        // 8 KiB: one operand, one K block
-constexpr int KPACK = MGX_CRT_KPACK;   // K blocks per pipeline stage
-constexpr int STAGE_BYTES = 2 * KPACK * SLAB;
-constexpr int STAGES = (232448 - 1280) / STAGE_BYTES;   // 227 KiB of shared memory per CTA
+// K blocks per pipeline stage.  Shorter stages cost more than the deeper ring gives: pairs, K = N =
+// 16384, 51.4 ms with 4 stages of 4 K blocks, 55.9 with 8 of 2, 67.0 with 16 of 1.
+constexpr int KPACK = 4;
 constexpr int EPI_WARPS = 16;          // four per TMEM lane quarter, 64 columns of either accumulator each
 constexpr int THREADS = (2 + EPI_WARPS) * 32;
 constexpr int NONFINITE = 0x7fffffff;
 constexpr int OUT_TILE_BYTES = TILE * TILE;   // one residue byte per output
-#ifndef MGX_CRT_RASTER
-#define MGX_CRT_RASTER 16
-#endif
-constexpr int RASTER = MGX_CRT_RASTER;
-
-static_assert(STAGES >= 2 && STAGES <= 8, "pipeline depth");
+constexpr int RASTER = 16;             // tile rows that sweep the columns together
 
 __constant__ int c_moduli[MAXQ] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
 static const int h_moduli[MAXQ] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
@@ -574,6 +562,9 @@ __device__ __forceinline__ uint64_t sw32_desc(uint32_t smem_addr)
 // kind::i8 instruction descriptor: D s32, A s8, B s8, both K-major, M = 128, N = 256.
 constexpr uint32_t IDESC_S8_128x256 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) |
                                       ((uint32_t)(128 >> 4) << 24);
+// The same for a pair of CTAs, M = 256: 128 rows of each.
+constexpr uint32_t IDESC_S8_256x256 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) |
+                                      ((uint32_t)(256 >> 4) << 24);
 
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
 {
@@ -615,7 +606,8 @@ __device__ __forceinline__ uint32_t mod_p_acc(uint32_t g, uint32_t p, uint32_t M
 struct GemmParams {
     const uint8_t *ra, *rb;   // residue slabs [modulus][tile][K block][256 x 32 B], at the block's first tile
     uint8_t *rc;              // output residues [modulus][tile row][tile column][64 KiB], at the block's first tile
-    size_t ra_mod, rb_mod, rc_mod;
+    size_t a_slabs, b_slabs, rc_mod;       // slabs of a modulus, bytes of its residue plane
+    CUtensorMap ma, mb;                    // pairs: the slabs of A and B as {256 words, 8, slabs}
     int tiles_m, tiles_n;     // tiles of this block of the product
     int rc_tile_ld;           // tiles per row of the residue planes (the whole product's)
     int kblocks, q;
@@ -628,25 +620,108 @@ struct GemmParams {
     uint32_t bias[MAXQ];      // p floor(2^31 / p), for mod_p_acc
 };
 
+// Shared memory of a CTA.  Alone: whole A and B slabs, 3 stages of 64 KiB.  As one of a pair: its own A
+// slabs and half of the pair's B slabs, 4 stages of 48 KiB.
+template <bool PAIR>
+struct Ring {
+    static constexpr int B_SLAB = PAIR ? SLAB / 2 : SLAB;
+    static constexpr int STAGE_BYTES = KPACK * (SLAB + B_SLAB);
+    static constexpr int STAGES = PAIR ? 4 : 3;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+};
+
 // Work item w: modulus w / (tiles), then groups of RASTER tile rows sweeping the columns
 // together (the group's rows of A stay in L2 while each column tile of B is read once per group).
+// tm: tile row, or pair of tile rows.
+template <bool PAIR>
 __device__ __forceinline__ void item_of(const GemmParams &p, int w, int &l, int &tm, int &tn, int &ks)
 {
+    constexpr int GROUP = PAIR ? RASTER / 2 : RASTER;
     ks = w % p.ksplit;       // K slice (consecutive items: the same tile's slices)
     w /= p.ksplit;
-    const int per = p.tiles_m * p.tiles_n;
+    const int rows = PAIR ? (p.tiles_m + 1) / 2 : p.tiles_m;
+    const int per = rows * p.tiles_n;
     l = w / per;
     const int t = w - l * per;
-    const int per_group = RASTER * p.tiles_n;
+    const int per_group = GROUP * p.tiles_n;
     const int g = t / per_group, r = t % per_group;
-    const int first = g * RASTER;
-    const int gsize = min(p.tiles_m - first, RASTER);
+    const int first = g * GROUP;
+    const int gsize = min(rows - first, GROUP);
     tm = first + r % gsize;
     tn = r / gsize;
 }
 
+// ---------------------------------------------------------------- CTA pairs
+__device__ __forceinline__ void cluster_sync()
+{
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Arrives on the barrier at `bar`'s offset in CTA `rank` of the cluster.
+__device__ __forceinline__ void mbar_arrive_remote(uint64_t *bar, uint32_t rank)
+{
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\t"
+        "mapa.shared::cluster.u32 a, %0, %1;\n\t"
+        "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(bar)),
+        "r"(rank)
+        : "memory");
+}
+
+// TMA box of this CTA, from this GPU's own memory into this CTA's shared memory, which completes on the
+// barrier at `bar`'s offset in the first CTA of the pair (bit 24 of the address is the CTA's rank).
+__device__ __forceinline__ void pair_load(void *dst, const CUtensorMap *map, int row, int slab, uint64_t *bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 "
+        "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(row), "r"(slab), "r"(smem_u32(bar) & 0xFEFFFFFFu)
+        : "memory");
+}
+
+// Commit of the issuer's MMAs to a barrier (of both CTAs of a pair).
+template <bool PAIR>
+__device__ __forceinline__ void commit(uint64_t *bar)
+{
+    if (PAIR)
+        asm volatile(
+            "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                smem_u32(bar)),
+            "h"((uint16_t)3)
+            : "memory");
+    else
+        tc_commit(bar);
+}
+
+template <bool PAIR>
+__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate)
+{
+    if (PAIR)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+            "l"(adesc), "l"(bdesc), "r"(IDESC_S8_256x256), "r"(accumulate)
+            : "memory");
+    else
+        tc_mma_i8(tmem_d, adesc, bdesc, IDESC_S8_128x256, accumulate);
+}
+
+// PAIR: two CTAs of a cluster work on two tile rows of one tile column.  Each copies its own A and half
+// of the B slabs, and the first CTA issues tcgen05 cta_group::2 MMAs (M = 256) that read both CTAs'
+// shared memory, so a CTA takes 12 KiB per K block from L2 instead of 16, reads half of B from its
+// shared memory, and a fourth stage fits.  The copies are TMA boxes because only those can complete on
+// the other CTA's barrier: the second CTA's bytes count on the first one's, and nothing relays them
+// (a relaying warp costs 1.5% at 4096, 15% if it releases at cluster scope).  At the power limit the
+// chip trades the saved energy for clock and utilisation -- residue products alone, 15 moduli, run
+// back to back at 1 kW: 2927 -> 2997 TOP/s at N = 16384 (tensor pipe busy 89% -> 92%), 2713 -> 2814 at
+// 4096, 2185 -> 2311 at 2048.
+template <bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ GemmParams p)
 {
+    using G = Ring<PAIR>;
+    constexpr int STAGES = G::STAGES, STAGE_BYTES = G::STAGE_BYTES, B_SLAB = G::B_SLAB;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                             ~uintptr_t(1023));
@@ -658,7 +733,9 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int items = p.q * p.tiles_m * p.tiles_n * p.ksplit;
+    const int items = p.q * (PAIR ? (p.tiles_m + 1) / 2 : p.tiles_m) * p.tiles_n * p.ksplit;
+    const int rank = PAIR ? (int)(blockIdx.x & 1) : 0;
+    const int first = PAIR ? blockIdx.x >> 1 : blockIdx.x, step = PAIR ? gridDim.x >> 1 : gridDim.x;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -667,19 +744,27 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
         }
         for (int h = 0; h < 2; ++h) {
             mbar_init(&acc_full[h], 1);
-            mbar_init(&acc_empty[h], EPI_WARPS);
+            mbar_init(&acc_empty[h], PAIR ? 2 * EPI_WARPS : EPI_WARPS);
         }
         mbar_init(drain, 1);
         fence_barrier_init();
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(512)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                         "r"(512)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                         "r"(512)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync();  // both CTAs' barriers and TMEM are set up
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();  // the set-up above overlaps the end of the previous kernel
@@ -693,11 +778,10 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
             int armed[STAGES];
             for (int s = 0; s < STAGES; ++s) armed[s] = -1;
             bool ok = true;
-            for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+            for (int w = first; w < items && ok; w += step) {
                 int l, tm, tn, ks;
-                item_of(p, w, l, tm, tn, ks);
+                item_of<PAIR>(p, w, l, tm, tn, ks);
                 const int kb_begin = ks * p.kb_split, kb_end = min(p.kblocks, kb_begin + p.kb_split);
-#if MGX_CRT_LOCKSTEP
                 // Soft lockstep: CTAs that share an operand tile read it from L2 only while they
                 // stay within a few microseconds of each other, so every producer waits at each
                 // new item until all CTAs have started theirs -- or 20 us, then goes on anyway.
@@ -705,28 +789,40 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
                 // share the GPU just wait out the 20 us).
                 if (p.sync) {
                     atomicAdd(p.sync, 1u);
-                    const unsigned int target = (unsigned int)min((long long)(w / gridDim.x + 1) * gridDim.x,
-                                                                  (long long)items);
+                    const unsigned int target =
+                        (unsigned int)(min((long long)(w / step + 1) * step, (long long)items) * (PAIR ? 2 : 1));
                     const unsigned long long t0 = global_ns();
                     while (*reinterpret_cast<volatile unsigned int *>(p.sync) < target &&
                            global_ns() - t0 < 20000ull)
                         __nanosleep(64);
                 }
-#endif
-                const uint8_t *ga = p.ra + (size_t)l * p.ra_mod + (size_t)tm * p.kblocks * SLAB;
-                const uint8_t *gb = p.rb + (size_t)l * p.rb_mod + (size_t)tn * p.kblocks * SLAB;
+                // (the second half of an odd last pair loads the last tile row again and stores nothing)
+                const int row = PAIR ? min(2 * tm + rank, p.tiles_m - 1) : tm;
+                const size_t sa0 = (size_t)l * p.a_slabs + (size_t)row * p.kblocks;
+                const size_t sb0 = (size_t)l * p.b_slabs + (size_t)tn * p.kblocks;
                 for (int kb0 = kb_begin; kb0 < kb_end; kb0 += KPACK) {
                     if (!mbar_wait_bounded(&empty[stage], phase ^ 1u, p.status, kDevTimeoutEmpty)) {
                         ok = false;
                         break;
                     }
                     const int nkb = min(KPACK, kb_end - kb0);
-                    const uint32_t bytes = (uint32_t)(nkb * SLAB);
-                    unsigned char *sa = smem + stage * STAGE_BYTES;
-                    mbar_arrive_expect_tx(&full[stage], 2u * bytes);
-                    armed[stage] = (int)phase;
-                    bulk_load(sa, ga + (size_t)kb0 * SLAB, bytes, &full[stage]);
-                    bulk_load(sa + KPACK * SLAB, gb + (size_t)kb0 * SLAB, bytes, &full[stage]);
+                    unsigned char *sa = smem + stage * STAGE_BYTES, *sb = sa + KPACK * SLAB;
+                    if (PAIR) {
+                        // Whole boxes, also where the K range ends inside one.  Both CTAs' copies arrive on
+                        // the first CTA's barrier, which expects the bytes of both.
+                        if (rank == 0) {
+                            mbar_arrive_expect_tx(&full[stage], 2u * STAGE_BYTES);
+                            armed[stage] = (int)phase;
+                        }
+                        pair_load(sa, &p.ma, 0, (int)(sa0 + kb0), &full[stage]);
+                        pair_load(sb, &p.mb, 4 * rank, (int)(sb0 + kb0), &full[stage]);
+                    } else {
+                        const uint32_t bytes = (uint32_t)(nkb * SLAB);
+                        mbar_arrive_expect_tx(&full[stage], 2u * bytes);
+                        armed[stage] = (int)phase;
+                        bulk_load(sa, p.ra + (sa0 + kb0) * SLAB, bytes, &full[stage]);
+                        bulk_load(sb, p.rb + (sb0 + kb0) * SLAB, bytes, &full[stage]);
+                    }
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1u;
@@ -745,12 +841,12 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
         // accumulator before the other's costs power (16384^3: 54.3 ms against 51.7).  Against one
         // hand-over of both accumulators after the whole drain (5,000 idle of 33,800 cycles per item at
         // K = 3008): 8192 x 8192 x 1024 1.60 -> 1.49 ms, 4096^3 1.14 -> 1.12, 16384^3 51.2 -> 50.8.
-        if (lane == 0) {
+        if (lane == 0 && rank == 0) {
             int stage = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
             const uint32_t smem_base = smem_u32(smem);
-            for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+            for (int w = first; w < items && ok; w += step) {
                 const int kb_begin = (w % p.ksplit) * p.kb_split, kb_end = min(p.kblocks, kb_begin + p.kb_split);
                 // MMAs over the stage at `st` that starts at K block kb, of accumulators h0 .. h1
                 auto issue = [&](int st, int kb, bool lo, bool hi) {
@@ -761,11 +857,9 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
                     for (int j = 0; j < KPACK; ++j) {
                         if (j < nkb) {
                             const uint32_t acc = (kb + j > kb_begin) ? 1u : 0u;
-                            const uint64_t bj = b0 + (uint64_t)((j * SLAB) >> 4);
-                            if (lo) tc_mma_i8(tmem_base, a0 + (uint64_t)((j * SLAB) >> 4), bj, IDESC_S8_128x256, acc);
-                            if (hi)
-                                tc_mma_i8(tmem_base + 256, a0 + (uint64_t)((j * SLAB + SLAB / 2) >> 4), bj,
-                                          IDESC_S8_128x256, acc);
+                            const uint64_t bj = b0 + (uint64_t)((j * B_SLAB) >> 4);
+                            if (lo) mma_i8<PAIR>(tmem_base, a0 + (uint64_t)((j * SLAB) >> 4), bj, acc);
+                            if (hi) mma_i8<PAIR>(tmem_base + 256, a0 + (uint64_t)((j * SLAB + SLAB / 2) >> 4), bj, acc);
                         }
                     }
                 };
@@ -775,14 +869,19 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
                         ph ^= 1u;
                     }
                 };
+                auto wait_stage = [&](int st, uint32_t ph) {
+                    const bool got = mbar_wait_bounded(&full[st], ph, p.status, kDevTimeoutFull);
+                    tc_fence_after();
+                    return got;
+                };
                 if (!mbar_wait_bounded(&acc_empty[0], acc_phase ^ 1u, p.status, kDevTimeoutAcc)) break;
                 tc_fence_after();
                 int kb0 = kb_begin, ahead = 0, st = stage;
                 uint32_t ph = phase;
-                while (ok && ahead < STAGES && kb0 < kb_end && !mbar_try_wait(&acc_empty[1], acc_phase ^ 1u)) {
-                    ok = mbar_wait_bounded(&full[st], ph, p.status, kDevTimeoutFull);
+                while (ok && ahead < STAGES && kb0 < kb_end &&
+                       !mbar_try_wait(&acc_empty[1], acc_phase ^ 1u)) {
+                    ok = wait_stage(st, ph);
                     if (!ok) break;
-                    tc_fence_after();
                     issue(st, kb0, true, false);
                     kb0 += KPACK;
                     ++ahead;
@@ -794,32 +893,29 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
                 tc_fence_after();
                 for (int i = 0; i < ahead; ++i) {
                     issue(stage, kb_begin + i * KPACK, false, true);
-                    tc_commit(&empty[stage]);  // frees the stage once these MMAs have read it
+                    commit<PAIR>(&empty[stage]);  // frees the stage once these MMAs have read it
                     next(stage, phase);
                 }
                 for (; kb0 < kb_end; kb0 += KPACK) {
-                    if (!mbar_wait_bounded(&full[stage], phase, p.status, kDevTimeoutFull)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
+                    ok = wait_stage(stage, phase);
+                    if (!ok) break;
                     if (kb0 + KPACK < kb_end) {
                         issue(stage, kb0, true, true);
                     } else {  // accumulator 0 is done first, and drains while the other's MMAs run
                         issue(stage, kb0, true, false);
-                        tc_commit(&acc_full[0]);
+                        commit<PAIR>(&acc_full[0]);
                         issue(stage, kb0, false, true);
                     }
-                    tc_commit(&empty[stage]);
+                    commit<PAIR>(&empty[stage]);
                     next(stage, phase);
                 }
                 if (ok) {
-                    if (kb_begin + ahead * KPACK >= kb_end) tc_commit(&acc_full[0]);  // all of it ran ahead
-                    tc_commit(&acc_full[1]);
+                    if (kb_begin + ahead * KPACK >= kb_end) commit<PAIR>(&acc_full[0]);  // all of it ran ahead
+                    commit<PAIR>(&acc_full[1]);
                 }
             }
             // Drain: all MMAs this thread issued have finished before TMEM is released.
-            tc_commit(drain);
+            commit<PAIR>(drain);
             mbar_wait_bounded(drain, 0, p.status, kDevTimeoutAcc);
         }
     } else {
@@ -828,12 +924,13 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
         const int c0 = (warp - 2) >> 2 << 1;  // first of its two 32-column chunks
         uint32_t acc_phase = 0;
         bool ok = true;
-        for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+        for (int w = first; w < items && ok; w += step) {
             int l, tm, tn, ks;
-            item_of(p, w, l, tm, tn, ks);
+            item_of<PAIR>(p, w, l, tm, tn, ks);
+            const int row = PAIR ? 2 * tm + rank : tm;
             const uint32_t pm = (uint32_t)c_moduli[l], M = p.barrett[l], bias = p.bias[l];
             uint8_t *dst = p.rc + (size_t)ks * p.rc_slice + (size_t)l * p.rc_mod +
-                           ((size_t)tm * p.rc_tile_ld + tn) * OUT_TILE_BYTES + (size_t)(qd * 32) * 256 + lane * 8;
+                           ((size_t)row * p.rc_tile_ld + tn) * OUT_TILE_BYTES + (size_t)(qd * 32) * 256 + lane * 8;
 #pragma unroll 1
             for (int h = 0; h < 2; ++h) {
                 bool got = true;
@@ -851,7 +948,13 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
                 tmem_wait_ld();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[h]);
+                if (lane == 0) {
+                    if (PAIR && rank == 1)
+                        mbar_arrive_remote(&acc_empty[h], 0);
+                    else
+                        mbar_arrive(&acc_empty[h]);
+                }
+                if (PAIR && row >= p.tiles_m) continue;
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
                     uint32_t pk[8];
@@ -875,7 +978,13 @@ __global__ void __launch_bounds__(THREADS, 1) crt_gemm(const __grid_constant__ G
     __syncthreads();
     tc_fence_after();
     __syncwarp();
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+    if (PAIR) cluster_sync();  // neither CTA leaves while the other may still reach its memory
+    if (warp == 1) {
+        if (PAIR)
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+        else
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+    }
 }
 
 // ---------------------------------------------------------------- CRT recombination
@@ -1272,6 +1381,7 @@ int crt_split_impl(const double *A, const double *B, int m, int n, int k, int ld
 // [c0, c0 + n), r0 and c0 multiples of 256.
 struct CrtView {
     const uint8_t *ra, *rb;
+    size_t a_slab0, b_slab0;  // slabs before ra, rb in the workspace
     uint8_t *rc;
     const int *sg, *tu;
     int m, n, tiles_m, tiles_n;
@@ -1283,6 +1393,8 @@ CrtView crt_view(const CrtLayout &L, unsigned char *ws, int r0, int c0, int m, i
     const int tm0 = r0 / crt::TILE, tn0 = c0 / crt::TILE;
     v.ra = ws + L.ra + (size_t)tm0 * L.kblocks * crt::SLAB;
     v.rb = ws + L.rb + (size_t)tn0 * L.kblocks * crt::SLAB;
+    v.a_slab0 = (size_t)tm0 * L.kblocks;
+    v.b_slab0 = (size_t)tn0 * L.kblocks;
     v.rc = ws + L.rc + ((size_t)tm0 * L.tiles_n + tn0) * crt::OUT_TILE_BYTES;
     v.sg = reinterpret_cast<const int *>(ws + L.sg) + r0;
     v.tu = reinterpret_cast<const int *>(ws + L.tu) + c0;
@@ -1302,8 +1414,8 @@ int crt_products_impl(const crt::Consts &K, const CrtLayout &L, const CrtView &v
     p.ra = v.ra;
     p.rb = v.rb;
     p.rc = v.rc;
-    p.ra_mod = L.ra_mod;
-    p.rb_mod = L.rb_mod;
+    p.a_slabs = L.ra_mod / crt::SLAB;
+    p.b_slabs = L.rb_mod / crt::SLAB;
     p.rc_mod = L.rc_mod;
     p.tiles_m = v.tiles_m;
     p.tiles_n = v.tiles_n;
@@ -1318,7 +1430,6 @@ int crt_products_impl(const crt::Consts &K, const CrtLayout &L, const CrtView &v
         p.barrett[l] = K.barrett[l];
         p.bias[l] = (uint32_t)crt::h_moduli[l] * (0x80000000u / (uint32_t)crt::h_moduli[l]);
     }
-    const int smem = crt::STAGES * crt::STAGE_BYTES + 1024 + 256;
     const long long items = (long long)K.q * v.tiles_m * v.tiles_n * L.ksplit;
     if (items <= 0) return MGX_SUCCESS;
     if (items > 0x7fffffffll) {
@@ -1335,8 +1446,27 @@ int crt_products_impl(const crt::Consts &K, const CrtLayout &L, const CrtView &v
         MGX_HOST_CHECK(cudaMemsetAsync(sync, 0, sizeof(unsigned int), stream));
         p.sync = sync;
     }
-    MGX_HOST_CHECK(cudaFuncSetAttribute(crt::crt_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    MGX_HOST_CHECK(mgx_launch_dependent(crt::crt_gemm, dim3((unsigned)grid), crt::THREADS, smem, stream, p));
+    // CTA pairs where their rounds of items are no more than single CTAs' (an odd last tile row makes
+    // half a pair idle) and four rounds or more pay for the pairs' setup: 1333 x 2011 x 1777, 5 rounds,
+    // 143 us against 147 alone; 1024^3, 2 rounds, 62.9 against 62.5.
+    const long long pairs = (long long)K.q * ((v.tiles_m + 1) / 2) * v.tiles_n * L.ksplit, slots = sms / 2;
+    if (slots > 0 && pairs >= 4 * slots && (pairs + slots - 1) / slots <= (items + sms - 1) / sms) {
+        int rc = mgx_encode_tmap_3d(&p.ma, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, v.ra, 256, 8, K.q * p.a_slabs - v.a_slab0,
+                                    1024, crt::SLAB, 256, 8, crt::KPACK, CU_TENSOR_MAP_SWIZZLE_NONE);
+        if (rc == MGX_SUCCESS)
+            rc = mgx_encode_tmap_3d(&p.mb, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, v.rb, 256, 8,
+                                    K.q * p.b_slabs - v.b_slab0, 1024, crt::SLAB, 256, 4, crt::KPACK,
+                                    CU_TENSOR_MAP_SWIZZLE_NONE);
+        if (rc != MGX_SUCCESS) return rc;
+        constexpr int smem = crt::Ring<true>::SMEM_BYTES;
+        MGX_HOST_CHECK(cudaFuncSetAttribute(crt::crt_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        MGX_HOST_CHECK(mgx_launch_dependent_cluster(crt::crt_gemm<true>, dim3(2u * (unsigned)slots), crt::THREADS, smem,
+                                                    stream, 2, p));
+        return MGX_SUCCESS;
+    }
+    constexpr int smem = crt::Ring<false>::SMEM_BYTES;
+    MGX_HOST_CHECK(cudaFuncSetAttribute(crt::crt_gemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    MGX_HOST_CHECK(mgx_launch_dependent(crt::crt_gemm<false>, dim3((unsigned)grid), crt::THREADS, smem, stream, p));
     return MGX_SUCCESS;
 }
 
