@@ -7,10 +7,11 @@
 // 1965 MHz); the design keeps the four sub-partitions of all SMs equally busy.
 //   * Work is cut in units of 8 columns of a 64-row band.  Every sub-partition owns 16 rows of the
 //     band and all of the tile's columns, so a tile of any width up to 128 columns loads the four
-//     pipes equally and its time is proportional to its width.  The CTAs' shares of a product can then
+//     pipes equally and its time is proportional to its width (a last band of up to 32 rows is
+//     spread over them by columns, see COST).  The CTAs' shares of a product can then
 //     be equal to within one unit (Walk), whatever the shape.  Against whole 128 x 128 tiles dealt
-//     to the SMs: N = 256 (4 tiles on 148 SMs) 39 -> 8.4 us, N = 1024 (64 tiles) 145 -> 69 us,
-//     1024 x 4096 x 2048 (256 tiles: 1.73 waves paid as 2) 614 -> 493 us, N = 8192 35.1 -> 35.9
+//     to the SMs: N = 256 (4 tiles on 148 SMs) 39 -> 7.5 us, N = 1024 (64 tiles) 145 -> 67 us,
+//     1024 x 4096 x 2048 (256 tiles: 1.73 waves paid as 2) 614 -> 493 us, N = 8192 35.1 -> 36.6
 //     TFLOP/s.
 //   * warpgroup 0 (producer, one lane): TMA 2D loads of A (BM x 32 doubles) and B (32 x up to 128)
 //     into a ring of 128-byte swizzled tiles, each stage guarded by a full/empty mbarrier pair.  No
@@ -30,6 +31,7 @@
 #include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 
 #include "mgx_common.cuh"
 
@@ -50,6 +52,7 @@ constexpr int THREADS = (CWARPS + PRODUCER_WARPS) * 32;   // 640 = 5 warpgroups
 // 128 x 32 + 512 x 112 = 61440 = 640 x 96.  The host refuses to launch unless the compiled
 // kernel has exactly LAUNCH_REGS registers per thread, so the split always adds up.
 constexpr int LAUNCH_REGS = 96, PRODUCER_REGS = 32, CONSUMER_REGS = 112;
+static_assert(CWARPS == 16 && BM == 64, "the warps' split of a tile");
 static_assert(PRODUCER_WARPS * 32 * PRODUCER_REGS + CWARPS * 32 * CONSUMER_REGS == THREADS * LAUNCH_REGS,
               "register split must equal the launch budget");
 
@@ -62,6 +65,13 @@ constexpr int STAGE_BYTES = A_STAGE_BYTES + 8 * B_BOX_BYTES;
 constexpr int STAGES = 4;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 constexpr int GROUP_M = 1024 / BM;           // stream-K raster groups of 1024 rows
+// A last band of at most 16 or 32 rows computes one or two 16-row strips, spread over all four
+// sub-partitions.  Its units then cost less by this measure, against COST for a whole band's; more than
+// a quarter and a half of it, because a warp has fewer units to hide its loads behind.  Sizes measured
+// with 2 and 4, 3 and 5, 4 and 6 of 8: 1040 x 4096 x 4096 1459, 991, 1008 us (1043 with whole bands
+// only), 1056 x 2048 x 4096 602, 505, 521 (526), 80 x 4096 x 4096 144, 128, 120 (143).  One band alone,
+// 8192 x 8192: 16 rows 279 -> 104 us, 32 rows 279 -> 189.
+constexpr int COST = 8, COST_1 = 3, COST_2 = 5;
 
 struct Params {
     double *C;
@@ -76,10 +86,14 @@ struct Params {
     int tiles_n;        // ceil(ucols / tile_units)
     int kblocks;        // K blocks of the whole reduction
     int skew;           // units that starting another band costs a CTA (see Walk)
+    int strips_last;    // log2 of the 16-row strips of the last band that are computed: 0, 1 or 2
+    int w_full, w_last; // what a unit of a band, and of the last band, costs (see Walk)
+    long long length;   // the product's length by that measure, and its part per CTA
+    long long share;
+    int share_rem;      // length - share x grid
+    long long sk_full;  // stream-K: K-block units of the tiles that cost w_full
     int panel_kb;       // > 0: SUMMA panels of so many K blocks; the running sum takes each panel's product
                         // with one rounding
-    int streamk;        // stream-K: CTA c takes the K-block units [c U / G, (c + 1) U / G) of all
-                        // U = tiles x kblocks, G = gridDim.x
     unsigned long long *sk_tickets;  // stream-K: one arrival ticket per tile and consumer warp
     unsigned long long sk_epoch;     // stream-K: this launch's ticket tag (a ticket of another tag counts 0)
     double *sk_partial; // stream-K: two partial accumulators per CTA (its first and last segment)
@@ -93,22 +107,34 @@ struct Params {
 // One piece of work: units [u0, u0 + units) of a band over K blocks [kb_begin, kb_end).
 struct Item {
     int band, u0, units, kb_begin, kb_end, slice;
-    int tile;  // stream-K: the tile this is a piece of
+    int strips;  // log2 of the 16-row strips that are computed
+    int tile;    // stream-K: the tile this is a piece of
 };
 
-// Tile coordinates of raster position `tile`: groups of 1024 rows sweep the columns together.
+// Tile coordinates of raster position `tile`: groups of 1024 rows sweep the columns together; the
+// tiles of a last band that costs less come after all others.
 __device__ __forceinline__ void tile_coords(const Params &p, int tile, int &tm, int &tn)
 {
+    const int bands = p.w_last < p.w_full ? p.bands - 1 : p.bands;
+    if (tile >= bands * p.tiles_n) {
+        tm = bands;
+        tn = tile - bands * p.tiles_n;
+        return;
+    }
     const int per_group = GROUP_M * p.tiles_n;
     const int group = tile / per_group;
     const int first_m = group * GROUP_M;
-    const int gsize = min(p.bands - first_m, GROUP_M);
+    const int gsize = min(bands - first_m, GROUP_M);
     const int r = tile % per_group;
     tm = first_m + r % gsize;
     tn = r / gsize;
 }
 
-__device__ __forceinline__ long long sk_begin(long long c, long long U, long long G) { return c * U / G; }
+// c U / G, where CTA c's share of a length U begins (U = share x G + share_rem).
+__device__ __forceinline__ long long sk_begin(const Params &p, unsigned c)
+{
+    return c * p.share + c * (unsigned)p.share_rem / gridDim.x;
+}
 
 // CTA whose share holds unit u (sk_begin(c) <= u < sk_begin(c + 1)).
 __device__ __forceinline__ int sk_owner(long long u, long long U, long long G)
@@ -116,56 +142,87 @@ __device__ __forceinline__ int sk_owner(long long u, long long U, long long G)
     return (int)(((u + 1) * G + U - 1) / U - 1);
 }
 
-// The work of one CTA, shared by the producer and the consumers.
-//   Regular: an equal share of the units of all (band, K slice) rows, in that order, cut into pieces
-//   no wider than a tile.  A share that runs on into another band works on two narrower pieces,
-//   which load A twice and leave some warps without a unit, so each row is given `skew`
-//   virtual units at its start that carry no work.
-//   Stream-K: the pieces of consecutive tiles' K ranges in this CTA's share of all K-block units.
+// Stream-K units are the K blocks of the tiles, in raster order.  They cost w_full each, those of a last
+// band of one or two strips w_last; where a unit starts on that scale, and the whole product's length.
+__device__ __forceinline__ long long sk_start(const Params &p, long long x)
+{
+    return x < p.sk_full ? x * p.w_full : p.sk_full * p.w_full + (x - p.sk_full) * p.w_last;
+}
+// The first unit that starts at `pos` or later.
+__device__ __forceinline__ long long sk_unit(const Params &p, long long pos)
+{
+    const long long rest = pos - p.sk_full * p.w_full;
+    if (p.w_full == 1) return pos;
+    return rest <= 0 ? (pos + p.w_full - 1) / p.w_full : p.sk_full + (rest + p.w_last - 1) / p.w_last;
+}
+
+// The work of one CTA, shared by the producer and the consumers: the units that start in its equal
+// share of the product's length.
+//   Regular: the units of all (band, K slice) rows, in that order, cut into pieces no wider than a
+//   tile.  A share that runs on into another band works on two narrower pieces, which load A
+//   twice and leave some warps without a unit, so each row is given `skew` virtual units at its
+//   start that carry no work.
+//   Stream-K: the pieces of consecutive tiles' K ranges.
+template <bool STREAMK, typename Unit>
 struct Walk {
-    long long u, u_end;  // the share's next unit and its end
+    Unit x, x_end;  // the share's next unit and its end
+
+    // (32 bits hold every position: a row's length is at most its part of C's bytes / 512)
+    static __device__ __forceinline__ unsigned row_unit(const Params &p, unsigned pos)
+    {
+        const unsigned len = (p.ucols + p.skew) * p.w_full, head = p.skew * p.w_full;
+        unsigned slice = 0;
+        if (p.ksplit > 1) {
+            const unsigned slice_len = (unsigned)p.length / (unsigned)p.ksplit;
+            slice = pos / slice_len;
+            pos -= slice * slice_len;
+        }
+        const unsigned band = min(pos / len, (unsigned)p.bands - 1u), off = pos - band * len;
+        const unsigned w = band == p.bands - 1u ? p.w_last : p.w_full;
+        unsigned first = off <= head ? 0u : off - head;
+        if (w > 1) first = (first + w - 1) / w;
+        return (slice * p.bands + band) * p.ucols + first;
+    }
 
     __device__ __forceinline__ void init(const Params &p)
     {
-        const long long U = p.streamk ? (long long)p.bands * p.tiles_n * p.kblocks
-                                      : (long long)p.bands * p.ksplit * (p.ucols + p.skew);
-        u = sk_begin(blockIdx.x, U, gridDim.x);
-        u_end = sk_begin(blockIdx.x + 1, U, gridDim.x);
+        const long long begin = sk_begin(p, blockIdx.x), end = sk_begin(p, blockIdx.x + 1);
+        if constexpr (STREAMK) {
+            x = sk_unit(p, begin);
+            x_end = sk_unit(p, end);
+        } else {
+            x = row_unit(p, (unsigned)begin);
+            x_end = row_unit(p, (unsigned)end);
+        }
     }
 
     __device__ __forceinline__ bool next(const Params &p, Item &it)
     {
-        if (u >= u_end) return false;
-        if (p.streamk) {
-            it.tile = (int)(u / p.kblocks);
+        if (x >= x_end) return false;
+        if constexpr (STREAMK) {
+            it.tile = (int)(x / p.kblocks);
             int tn;
             tile_coords(p, it.tile, it.band, tn);
             it.u0 = tn * p.tile_units;
             it.units = min(p.tile_units, p.ucols - it.u0);
             it.slice = 0;
-            it.kb_begin = (int)(u - (long long)it.tile * p.kblocks);
-            const long long left = u_end - u;
-            it.kb_end = (long long)(p.kblocks - it.kb_begin) < left ? p.kblocks : it.kb_begin + (int)left;
-            u += it.kb_end - it.kb_begin;
-            return true;
+            it.kb_begin = (int)(x - (long long)it.tile * p.kblocks);
+            it.kb_end = (int)min((long long)p.kblocks, it.kb_begin + x_end - x);
+            x += it.kb_end - it.kb_begin;
+        } else {
+            const unsigned row = x / (unsigned)p.ucols;
+            const int off = (int)(x - row * p.ucols);
+            const int run = min(p.ucols - off, (int)(x_end - x));  // the row's units in this share
+            const int pieces = (run + TILE_UNITS - 1) / TILE_UNITS;
+            it.slice = p.ksplit > 1 ? row / p.bands : 0;
+            it.band = row - it.slice * p.bands;
+            it.u0 = off;
+            it.units = (run + pieces - 1) / pieces;
+            it.kb_begin = it.slice * p.kb_split;
+            it.kb_end = min(p.kblocks, it.kb_begin + p.kb_split);
+            x += it.units;
         }
-        const int len = p.ucols + p.skew;
-        int row = (int)(u / len);
-        int off = (int)(u - (long long)row * len) - p.skew;
-        if (off < 0) {  // skip the row's virtual units
-            u -= off;
-            off = 0;
-            if (u >= u_end) return false;
-        }
-        const int run = (int)min((long long)(p.ucols - off), u_end - u);  // the row's units in this share
-        const int pieces = (run + TILE_UNITS - 1) / TILE_UNITS;
-        it.band = row % p.bands;
-        it.slice = row / p.bands;
-        it.u0 = off;
-        it.units = (run + pieces - 1) / pieces;
-        it.kb_begin = it.slice * p.kb_split;
-        it.kb_end = min(p.kblocks, it.kb_begin + p.kb_split);
-        u += it.units;
+        it.strips = it.band == p.bands - 1 ? p.strips_last : 2;
         return true;
     }
 };
@@ -277,7 +334,9 @@ __device__ __forceinline__ bool reduce_item(const Params &p, Consumer &c, int kb
     return true;
 }
 
-template <bool PANELS>
+// A kernel for each form, so that each is scheduled for itself: with stream-K's epilogue in the whole-K
+// kernel 2048 x 8192 x 2048 took 1930 us against 1885, N = 1024 68.5 against 66.8, N = 256 5.04 against 4.77.
+template <bool PANELS, bool STREAMK>
 __global__ void __launch_bounds__(THREADS, 1)
     dgemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Params p)
 {
@@ -308,7 +367,10 @@ __global__ void __launch_bounds__(THREADS, 1)
     pdl_wait();
     pdl_trigger();
 
-    Walk walk;
+    // The panel form's two accumulator sets leave it few registers, and its speed depends on what else is
+    // live: 3001 x 5002 x 4096 in panels of 512 takes 3496 us with 64-bit positions, 3565 with 32-bit
+    // ones.  The whole-K form is 1.5% faster with 32-bit ones at N = 256.
+    Walk<STREAMK, std::conditional_t<PANELS || STREAMK, long long, unsigned>> walk;
     walk.init(p);
     Item it;
 
@@ -359,7 +421,6 @@ __global__ void __launch_bounds__(THREADS, 1)
     c.empty = empty;
     c.smem_base = smem_u32(smem);
     c.lane = lane;
-    c.strip = cw & 3;  // warps cw, cw + 4, ... share a sub-partition and its 16 rows
     c.stage = 0;
     c.phase = 0;
 
@@ -394,10 +455,13 @@ __global__ void __launch_bounds__(THREADS, 1)
     };
 
     while (walk.next(p, it)) {
-        // this warp's part of the tile's units (the warps of a sub-partition share its pipe, so an
-        // uneven split does not unbalance anything)
-        const int per = (it.units + SUB_WARPS - 1) / SUB_WARPS;
-        c.u_first = (cw >> 2) * per;
+        // This warp's strip and part of the tile's units.  Warps cw, cw + 4, ... share a sub-partition:
+        // its 16 rows of a whole band, so an uneven split of the units does not unbalance anything.
+        // One or two strips are spread over all sub-partitions, a column's units over neighbours.
+        if (PANELS) it.strips = 2;  // (a variable one costs 1%; the host asks for no other)
+        c.strip = cw & ((1 << it.strips) - 1);
+        const int sharers = CWARPS >> it.strips, per = (it.units + sharers - 1) >> (4 - it.strips);
+        c.u_first = (cw >> it.strips) * per;
         const int nu = max(0, min(per, it.units - c.u_first));
 
         double acc[WARP_UNITS][4];
@@ -426,67 +490,66 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
                 for (int v = 0; v < 4; ++v) acc[j][v] = tot[j][v];
         }
-        if (p.streamk) {
-            if constexpr (!PANELS) {
-                // A tile whose K range spans several CTAs' shares is finished by the CTA that
-                // arrives last at its ticket: every piece's accumulator goes to that CTA's partial
-                // slot, and the last arrival adds the pieces in K order (p0 + p1) + p2 ... and
-                // stores C.  No CTA waits for another.
-                const long long U = (long long)p.bands * p.tiles_n * p.kblocks, NG = gridDim.x;
-                const long long t0 = (long long)it.tile * p.kblocks;
-                const int c0 = sk_owner(t0, U, NG), pieces = sk_owner(t0 + p.kblocks - 1, U, NG) - c0 + 1;
-                if (pieces == 1) {
+        if constexpr (STREAMK) {
+            // A tile whose K range spans several CTAs' shares is finished by the CTA that
+            // arrives last at its ticket: every piece's accumulator goes to that CTA's partial
+            // slot, and the last arrival adds the pieces in K order (p0 + p1) + p2 ... and
+            // stores C.  No CTA waits for another.
+            const long long U = p.length, NG = gridDim.x;
+            const long long t0 = (long long)it.tile * p.kblocks;
+            const int c0 = sk_owner(sk_start(p, t0), U, NG);
+            const int pieces = sk_owner(sk_start(p, t0 + p.kblocks - 1), U, NG) - c0 + 1;
+            if (pieces == 1) {
+                store_acc(acc, nu, p.beta_one, p.C, p.ldc, p.vec_store);
+            } else {
+                // Each consumer warp owns the same fragment of the tile in every piece, so it
+                // finishes that fragment on its own: a ticket per (tile, warp), and no barrier
+                // between the warps (a warp that gave up on a wait cannot block the others).
+                constexpr int NACC = WARP_UNITS * 4;
+                constexpr size_t PART = (size_t)CWARPS * 32 * NACC;  // doubles per partial slot
+                const int ct = threadIdx.x - PRODUCER_WARPS * 32;     // consumer thread 0..255
+                const int j = (int)blockIdx.x - c0;                    // this CTA's piece
+                const int slot = (t0 + it.kb_begin == sk_unit(p, sk_begin(p, blockIdx.x))) ? 0 : 1;
+                double(&af)[NACC] = reinterpret_cast<double(&)[NACC]>(acc);
+                const int na = nu * 4;
+                unsigned long long *ticket = p.sk_tickets + (size_t)it.tile * CWARPS + cw;
+                // The head piece is usually computed last (at the end of its CTA's share):
+                // when every later piece has taken its ticket, it finishes the tile without
+                // writing its own partial.
+                int last = 0;
+                if (j == 0) {
+                    if (lane == 0) last = ticket_count(ticket, p.sk_epoch) == pieces - 1;
+                    last = __shfl_sync(0xffffffffu, last, 0);
+                }
+                if (!last) {
+                    double *mine = p.sk_partial + ((size_t)blockIdx.x * 2 + slot) * PART;
+#pragma unroll
+                    for (int i = 0; i < NACC; ++i)
+                        if (i < na) __stcg(mine + (size_t)i * (CWARPS * 32) + ct, af[i]);
+                    __threadfence();
+                    __syncwarp();
+                    if (lane == 0) last = ticket_take(ticket, p.sk_epoch, p.status) == pieces - 1;
+                    last = __shfl_sync(0xffffffffu, last, 0);
+                }
+                if (last) {
+                    __threadfence();
+                    double tot_k[NACC];
+                    const int slot0 = (sk_unit(p, sk_begin(p, c0)) == t0) ? 0 : 1;
+                    const double *p0 = p.sk_partial + ((size_t)c0 * 2 + slot0) * PART;
+#pragma unroll
+                    for (int i = 0; i < NACC; ++i)
+                        tot_k[i] = j == 0 || i >= na ? af[i] : __ldcg(p0 + (size_t)i * (CWARPS * 32) + ct);
+                    for (int jj = 1; jj < pieces; ++jj) {
+                        // pieces after the first start their CTA's share: slot 0
+                        const double *pj = p.sk_partial + ((size_t)(c0 + jj) * 2) * PART;
+#pragma unroll
+                        for (int i = 0; i < NACC; ++i)
+                            if (i < na)
+                                tot_k[i] = tot_k[i] + (jj == j ? af[i] : __ldcg(pj + (size_t)i * (CWARPS * 32) + ct));
+                    }
+#pragma unroll
+                    for (int i = 0; i < NACC; ++i) af[i] = tot_k[i];
                     store_acc(acc, nu, p.beta_one, p.C, p.ldc, p.vec_store);
-                } else {
-                    // Each consumer warp owns the same fragment of the tile in every piece, so it
-                    // finishes that fragment on its own: a ticket per (tile, warp), and no barrier
-                    // between the warps (a warp that gave up on a wait cannot block the others).
-                    constexpr int NACC = WARP_UNITS * 4;
-                    constexpr size_t PART = (size_t)CWARPS * 32 * NACC;  // doubles per partial slot
-                    const int ct = threadIdx.x - PRODUCER_WARPS * 32;     // consumer thread 0..255
-                    const int j = (int)blockIdx.x - c0;                    // this CTA's piece
-                    const int slot = (t0 + it.kb_begin == sk_begin(blockIdx.x, U, NG)) ? 0 : 1;
-                    double(&af)[NACC] = reinterpret_cast<double(&)[NACC]>(acc);
-                    const int na = nu * 4;
-                    unsigned long long *ticket = p.sk_tickets + (size_t)it.tile * CWARPS + cw;
-                    // The head piece is usually computed last (at the end of its CTA's share):
-                    // when every later piece has taken its ticket, it finishes the tile without
-                    // writing its own partial.
-                    int last = 0;
-                    if (j == 0) {
-                        if (lane == 0) last = ticket_count(ticket, p.sk_epoch) == pieces - 1;
-                        last = __shfl_sync(0xffffffffu, last, 0);
-                    }
-                    if (!last) {
-                        double *mine = p.sk_partial + ((size_t)blockIdx.x * 2 + slot) * PART;
-#pragma unroll
-                        for (int i = 0; i < NACC; ++i)
-                            if (i < na) __stcg(mine + (size_t)i * (CWARPS * 32) + ct, af[i]);
-                        __threadfence();
-                        __syncwarp();
-                        if (lane == 0) last = ticket_take(ticket, p.sk_epoch, p.status) == pieces - 1;
-                        last = __shfl_sync(0xffffffffu, last, 0);
-                    }
-                    if (last) {
-                        __threadfence();
-                        double tot_k[NACC];
-                        const int slot0 = (sk_begin(c0, U, NG) == t0) ? 0 : 1;
-                        const double *p0 = p.sk_partial + ((size_t)c0 * 2 + slot0) * PART;
-#pragma unroll
-                        for (int i = 0; i < NACC; ++i)
-                            tot_k[i] = j == 0 || i >= na ? af[i] : __ldcg(p0 + (size_t)i * (CWARPS * 32) + ct);
-                        for (int jj = 1; jj < pieces; ++jj) {
-                            // pieces after the first start their CTA's share: slot 0
-                            const double *pj = p.sk_partial + ((size_t)(c0 + jj) * 2) * PART;
-#pragma unroll
-                            for (int i = 0; i < NACC; ++i)
-                                if (i < na)
-                                    tot_k[i] = tot_k[i] + (jj == j ? af[i] : __ldcg(pj + (size_t)i * (CWARPS * 32) + ct));
-                        }
-#pragma unroll
-                        for (int i = 0; i < NACC; ++i) af[i] = tot_k[i];
-                        store_acc(acc, nu, p.beta_one, p.C, p.ldc, p.vec_store);
-                    }
                 }
             }
         } else if (p.ksplit > 1)
@@ -709,8 +772,36 @@ static int launch_dgemm(const double *A, const double *B, double *C, int m, int 
     // one and 388 with two virtual units; N = 1024 75.3, 70.8, 69.1).  With shares of a few units the
     // virtual ones would take whole shares away, so they are left out there.
     p.skew = units >= 8ll * grid ? 2 : 0;
+    if (mode.streamk) grid = streamk_grid(m, n, k_len);
+    // A last band of one or two strips (not in the panel form, see its kernel).  Stream-K: a CTA without
+    // a unit would be counted among a tile's pieces, so shares are no shorter than the longest unit.
+    // Where every CTA has one unit at most the weights would only move units together: 80 x 512 x 1024
+    // 13.0 us without them, 13.6 with.
+    p.strips_last = 2;
+    p.w_full = p.w_last = 1;
+    const int strips = (m - (cut.bands - 1) * fp64::BM + 15) / 16;
+    if (strips <= 2 && !panels) {
+        const int w = strips == 1 ? fp64::COST_1 : fp64::COST_2;
+        const long long row = (long long)cut.tiles_n * p.kblocks;
+        const bool weigh = cut.bands == 1 ? false
+                           : mode.streamk ? row * ((cut.bands - 1) * fp64::COST + w) >= (long long)grid * fp64::COST
+                                          : units > sms;
+        if (weigh) {
+            p.w_full = fp64::COST;
+            p.w_last = w;
+        }
+        if (weigh || cut.bands == 1 || !mode.streamk) p.strips_last = strips - 1;
+    }
     if (mode.streamk) {
-        grid = streamk_grid(m, n, k_len);
+        p.sk_full = (long long)(p.w_last < p.w_full ? cut.bands - 1 : cut.bands) * cut.tiles_n * p.kblocks;
+        p.length = p.sk_full * p.w_full + ((long long)cut.bands * cut.tiles_n * p.kblocks - p.sk_full) * p.w_last;
+    } else {
+        p.length = slices * ((cut.bands - 1) * (long long)(cut.ucols + p.skew) * p.w_full + p.skew * p.w_full +
+                             (long long)cut.ucols * p.w_last);
+    }
+    p.share = p.length / grid;
+    p.share_rem = (int)(p.length - p.share * grid);
+    if (mode.streamk) {
         if (grid > 255) {  // arrivals per tile must fit a ticket's 8-bit count
             mgx_set_last_message("FP64 stream-K: grid of %d CTAs exceeds 255", grid);
             return MGX_E_UNSUPPORTED;
@@ -722,7 +813,6 @@ static int launch_dgemm(const double *A, const double *B, double *C, int m, int 
                                  pbytes + tbytes, mode.ws_bytes);
             return MGX_E_WORKSPACE;
         }
-        p.streamk = 1;
         p.sk_partial = reinterpret_cast<double *>(mode.ws);
         p.sk_tickets = reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(mode.ws) + pbytes);
         // a fresh tag per launch (56 bits, never 0: zeroed memory reads as no arrivals)
@@ -795,7 +885,9 @@ static int launch_dgemm(const double *A, const double *B, double *C, int m, int 
                                             tmA, tmB, p));
         return MGX_SUCCESS;
     };
-    if (rc == MGX_SUCCESS) rc = panels ? launch(fp64::dgemm_kernel<true>) : launch(fp64::dgemm_kernel<false>);
+    if (rc == MGX_SUCCESS) rc = panels           ? launch(fp64::dgemm_kernel<true, false>)
+                                : mode.streamk ? launch(fp64::dgemm_kernel<false, true>)
+                                               : launch(fp64::dgemm_kernel<false, false>);
     if (scratch) cudaFreeAsync(scratch, stream);
     if (rc != MGX_SUCCESS) return rc;
     MGX_HOST_CHECK(cudaGetLastError());
