@@ -550,6 +550,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
                     for (int i = 0; i < NACC; ++i) af[i] = tot_k[i];
                     store_acc(acc, nu, p.beta_one, p.C, p.ldc, p.vec_store);
+                    // a graph replays the launch with the same tag, which must find no arrivals
+                    if (lane == 0) atomicExch(ticket, 0ull);
                 }
             }
         } else if (p.ksplit > 1)
