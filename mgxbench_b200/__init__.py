@@ -207,7 +207,7 @@ def gemm_fp64(A, B, C, beta_one: bool = False, stream=None, ksplit: int = 1, wor
     m, k = A.shape
     n = B.shape[1]
     if ksplit == 0:
-        # stream-K over 64 x 128 tiles
+        # stream-K over tiles of 64 rows
         need = lib().mgx_fp64_streamk_workspace_size(m, n, k)
         ws = (workspace or _default_ws).get(need) if need else None
         return _check(lib().mgx_gemm_fp64_streamk(_ptr(A), _ptr(B), _ptr(C), m, n, k, _ld(A), _ld(B), _ld(C),

@@ -29,19 +29,20 @@ from pathlib import Path
 
 import numpy as np
 
-TILE_FP64 = 0          # native FP64 kernel (DMMA), 128 x 128 output tiles over the whole K range
+# The FP64 kernel cuts every product in equal shares per SM: the tile heights of 128 and 64 rows that
+# ids 0, 2-5 and 9-12 name (of the kernel that the packaged sweep measured) now run alike.
+TILE_FP64 = 0          # native FP64 kernel (DMMA), 128 rows, over the whole K range
 TILE_OZAKI_128 = 1     # Ozaki INT8 kernel, 128 x 128 output tiles over the whole K range
-# native FP64 kernel, 128 x 128 output tiles, K cut into 2 / 4 / 8 / 16 slices (split-K)
+# native FP64 kernel, 128 rows, K cut into 2 / 4 / 8 / 16 slices (split-K)
 TILE_FP64_K2, TILE_FP64_K4, TILE_FP64_K8, TILE_FP64_K16 = 2, 3, 4, 5
 # Ozaki INT8 kernel, 128 x 128 output tiles, K cut into 4 / 16 slices (split-K)
 TILE_OZAKI_K4, TILE_OZAKI_K16 = 6, 7
 # CRT form (Ozaki scheme II), 256 x 256 output tiles over the whole K range; its "splits" is the
 # modulus count
 TILE_CRT = 8
-# native FP64 kernel, 64 x 128 output tiles (twice the work items of the 128 x 128 tile), over the
-# whole K range or cut into 2 / 4 / 8 slices
+# native FP64 kernel, 64 rows, over the whole K range or cut into 2 / 4 / 8 slices
 TILE_FP64_T64, TILE_FP64_T64_K2, TILE_FP64_T64_K4, TILE_FP64_T64_K8 = 9, 10, 11, 12
-# native FP64 kernel, 64 x 128 output tiles, stream-K: every CTA an equal share of all tiles' K
+# native FP64 kernel, tiles of 64 rows, stream-K: every CTA an equal share of all tiles' K
 # blocks (its "ksplit" is 0)
 TILE_FP64_T64_SK = 13
 FP64_KSPLIT = {TILE_FP64: 1, TILE_FP64_K2: 2, TILE_FP64_K4: 4, TILE_FP64_K8: 8, TILE_FP64_K16: 16,

@@ -47,9 +47,8 @@ def _mat(r, c, kind, seed, e_range=0):
 
 
 def cfg1():
-    """The drop-in call (mgx_ab_multiply: 128 x 128 tiles, whole K), then every FP64 tile shape and
-    K-slice count measured (64 output tiles of 128 x 128 leave most of the 148 SMs idle), and the
-    one the learned cost model picks."""
+    """The drop-in call (mgx_ab_multiply: whole K), then every FP64 tile id and K-slice count of the
+    autotuner measured, and the one the learned cost model picks."""
     n = 1024
     A, B, C = _mat(n, n, 1, 11), _mat(n, n, 1, 12), torch.empty((n, n), dtype=torch.float64, device="cuda")
     peak = max(mgx.peak_fp64(k, 20000) for k in (3, 4))

@@ -81,9 +81,9 @@ inline std::string exe_dir()
 
 inline std::string default_model_path() { return exe_dir() + "/../mgxbench_b200/data/mlp_b200.json"; }
 
-// Tile ids of the candidates (mgxbench_b200.autotune): 0, 2, 3, 4, 5 are the FP64 kernel's
-// 128 x 128 tiles with the K range cut into 1, 2, 4, 8, 16 slices; 9, 10, 11, 12 its 64 x 128
-// tiles with 1, 2, 4, 8 slices and 13 its 64 x 128 tiles in the stream-K schedule (K slices 0);
+// Tile ids of the candidates (mgxbench_b200.autotune): 0, 2, 3, 4, 5 are the FP64 kernel with
+// tile_m 128 and the K range cut into 1, 2, 4, 8, 16 slices; 9, 10, 11, 12 with tile_m 64 and 1, 2,
+// 4, 8 slices (the kernel runs both alike) and 13 its stream-K schedule (K slices 0);
 // 1, 6, 7 are the Ozaki kernel with 1, 4, 16 slices; 8 is the CRT form (its "splits" is the
 // modulus count).
 inline int tile_ksplit(int tile)

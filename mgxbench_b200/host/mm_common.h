@@ -132,7 +132,7 @@ struct Workspace {
 inline int block_gemm(int form, int splits, int ksplit, Workspace &ws, const double *A, const double *B, double *C,
                       int m, int n, int k, int lda, int ldb, int ldc, int beta_one, cudaStream_t s, int tile_m = 128)
 {
-    if (form == kFp64 && ksplit == 0) {  // stream-K over 64 x 128 tiles
+    if (form == kFp64 && ksplit == 0) {  // stream-K over tiles of 64 rows
         const size_t need = mgx_fp64_streamk_workspace_size(m, n, k);
         void *w = ws.get(need);
         if (!w && need) return MGX_E_CUDA;
