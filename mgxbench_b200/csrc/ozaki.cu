@@ -163,18 +163,19 @@ __global__ void __launch_bounds__(T) ozaki_row_exp(const double *__restrict__ A,
 
 // grid (ceil(n/256), ychunks); each thread scans a run of rows of one column, 8 loads in flight; the
 // last block of each column group to arrive takes the exponents.
+// This and the digit passes read B or A before they wait for the kernel before them: it writes neither,
+// and they only start once all its blocks have seen their own predecessors complete.  Whole products, 8
+// slices: 1024^3 85.0 -> 79.3 us, 512^3 55.3 -> 51.9, 2048^3 261 -> 258.
 __global__ void __launch_bounds__(256) ozaki_col_max(const double *__restrict__ B, int k, int n, int ldb, const ColStats z,
                                                      int *__restrict__ eb, int *status)
 {
     __shared__ bool last;
-    pdl_wait();
-    pdl_trigger();
     const int j = blockIdx.x * 256 + threadIdx.x;
+    unsigned long long mx = 0;
     if (j < n) {
         const int rows_per = (k + gridDim.y - 1) / gridDim.y;
         const int r0 = blockIdx.y * rows_per;
         const int r1 = min(k, r0 + rows_per);
-        unsigned long long mx = 0;
         const unsigned long long *b = reinterpret_cast<const unsigned long long *>(B) + j;
         int r = r0;
         for (; r + 8 <= r1; r += 8) {
@@ -188,15 +189,17 @@ __global__ void __launch_bounds__(256) ozaki_col_max(const double *__restrict__ 
             const unsigned long long v = __ldg(b + (size_t)r * ldb) & 0x7fffffffffffffffull;
             mx = v > mx ? v : mx;
         }
-        if (mx) atomicMax(z.max + j, mx);
     }
+    pdl_wait();
+    pdl_trigger();
+    if (mx) atomicMax(z.max + j, mx);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = atomicAdd(z.arrived + blockIdx.x, 1u) == gridDim.y - 1;
     __syncthreads();
     if (!last || j >= n) return;
     __threadfence();
-    const unsigned long long mx = __ldcg(z.max + j);
+    mx = __ldcg(z.max + j);
     if (mx >= 0x7ff0000000000000ull) {
         eb[j] = NONFINITE_EXP;
         record_status(status, kDevNonFinite);
@@ -250,8 +253,6 @@ __global__ void __launch_bounds__(256) ozaki_split_a(const double *__restrict__ 
                                                      const int *__restrict__ ea, uint8_t *__restrict__ da)
 {
     __shared__ __align__(16) double tile[8][8][32];
-    pdl_wait();
-    pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int kb = blockIdx.y, row0 = blockIdx.x * 64 + warp * 8, r = lane >> 2, kq = lane & 3, row = row0 + r;
     {
@@ -266,6 +267,8 @@ __global__ void __launch_bounds__(256) ozaki_split_a(const double *__restrict__ 
         for (int i = 0; i < 8; ++i)
             tile[warp][i][(4 * q + ((j + (q >> 1) + 2 * (i & 1)) & 3)) * 2 + (lane & 1)] = v[i];
     }
+    pdl_wait();
+    pdl_trigger();
     int e = (row < m) ? ea[row] : 0;
     const bool live = e != NONFINITE_EXP;  // a live row holds finite values only
     if (!live) e = 0;
@@ -289,8 +292,6 @@ __global__ void __launch_bounds__(256) ozaki_split_b(const double *__restrict__ 
                                                      const int *__restrict__ eb, uint8_t *__restrict__ db)
 {
     __shared__ double tb[32][65];
-    pdl_wait();
-    pdl_trigger();
     const int n0 = blockIdx.x * 64, kb = blockIdx.y, k0 = kb * 32;
     {
         const int c = threadIdx.x & 63, kr = threadIdx.x >> 6;
@@ -301,6 +302,8 @@ __global__ void __launch_bounds__(256) ozaki_split_b(const double *__restrict__ 
 #pragma unroll
         for (int i = 0; i < 8; ++i) tb[kr + 4 * i][c] = v[i];
     }
+    pdl_wait();
+    pdl_trigger();
     const int r = threadIdx.x >> 2, kq = threadIdx.x & 3, col = n0 + r;   // tile row r % 128 = column of B
     int e = (col < n) ? eb[col] : 0;
     const bool live = e != NONFINITE_EXP;  // a live column holds finite values only
