@@ -359,8 +359,8 @@ MGX_API int mgx_mlp_adam_step(float *params, const float *grads, float *m, float
  * ------------------------------------------------------------------------------------------ */
 
 /* Returns the device memory the library keeps cached for its scratch (operand packing, the
- * host-buffer pipeline) on the current device: it synchronises the device, then releases the
- * cache.  Later calls allocate again.  No counterpart in MGXBench. */
+ * host-buffer pipeline) on the current device, and the constant check's page-locked buffers: it
+ * synchronises the device, then releases the cache.  Later calls allocate again.  No counterpart in MGXBench. */
 MGX_API int mgx_scratch_trim(void);
 
 /* Exercises the timeout path of the library's bounded device-side waits: a kernel waits on a

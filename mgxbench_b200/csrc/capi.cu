@@ -164,10 +164,13 @@ int mgx_scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream)
     return MGX_SUCCESS;
 }
 
+void mgx_validate_trim();  // validate.cu
+
 MGX_API int mgx_scratch_trim(void)
 {
     const int dev = current_device();
     if (dev < 0 || dev >= kMaxDevices) return MGX_E_CUDA;
+    mgx_validate_trim();
     cudaMemPool_t pool = nullptr;
     {
         std::lock_guard<std::mutex> lk(g_mu);

@@ -11,6 +11,7 @@
 #include <cfloat>
 #include <cstring>
 #include <cmath>
+#include <mutex>
 
 #include "mgx_common.cuh"
 
@@ -218,50 +219,96 @@ static double bits_to_double(unsigned long long b)
 
 namespace {
 
-// Page-locked memory the constant check's blocks write their findings to and the calling thread reads:
-// 32 KiB per host thread and device, given back when the thread ends, taken anew when the device's
-// context has changed since (a cudaDeviceReset freed it then).  With device accumulators, the call had
-// an allocation, a memset, a copy back through pageable memory and a free around its kernel.
-constexpr int kParts = 2048, kDevices = 64;
+// Page-locked buffers that the constant check's blocks write their findings to and the calling thread
+// reads.  A call takes an idle one of its context and hands it back once it has read it, so as many are
+// held as calls ever ran at once, at most kIdle of 32 KiB (mgx_scratch_trim frees them), and a thread's
+// end frees nothing: cudaFreeHost waits for all of the device's work.  Never destroyed: threads may
+// still check while the process exits.  A buffer whose context a cudaDeviceReset has ended is gone with
+// it and is never found again, as the context after it has another id; without an id (driver without the
+// call) nothing is kept.  With device accumulators instead, the call had an allocation, a memset, a
+// copy back through pageable memory and a free around its kernel.
+constexpr int kParts = 2048;
+constexpr int kIdle = 64;
 
-struct PartsBuffers {
-    struct Slot {
+class PartsPool {
+public:
+    struct Buffer {
         val::ConstPart *ptr;
         unsigned long long ctx;
-    } slot[kDevices] = {};
+    };
 
-    ~PartsBuffers()
+    int take(Buffer *out)
     {
-        int current = -1;
-        if (cudaGetDevice(&current) != cudaSuccess) return;
-        for (int d = 0; d < kDevices; ++d)
-            if (slot[d].ptr && cudaSetDevice(d) == cudaSuccess) {
-                if (mgx_context_id() == slot[d].ctx) cudaFreeHost(slot[d].ptr);
-                cudaSetDevice(current);
-            }
-    }
-
-    int take(val::ConstPart **out)
-    {
-        int d = 0;
-        MGX_HOST_CHECK(cudaGetDevice(&d));
-        if (d >= kDevices) {
-            mgx_set_last_message("constant validation: device %d is beyond %d", d, kDevices);
-            return MGX_E_UNSUPPORTED;
+        unsigned long long ctx = mgx_context_id();
+        if (ctx == 0) {  // a thread's first call: no context current yet
+            int d = 0;
+            MGX_HOST_CHECK(cudaGetDevice(&d));
+            MGX_HOST_CHECK(cudaSetDevice(d));
+            ctx = mgx_context_id();
         }
-        Slot &s = slot[d];
-        if (!s.ptr || mgx_context_id() != s.ctx) {
-            s.ptr = nullptr;
-            MGX_HOST_CHECK(cudaHostAlloc(reinterpret_cast<void **>(&s.ptr), kParts * sizeof(val::ConstPart),
-                                         cudaHostAllocPortable | cudaHostAllocMapped));
-            s.ctx = mgx_context_id();
+        if (ctx != 0) {
+            std::lock_guard<std::mutex> lk(mu_);
+            for (int i = count_ - 1; i >= 0; --i)
+                if (idle_[i].ctx == ctx) {
+                    *out = remove(i);
+                    return MGX_SUCCESS;
+                }
         }
-        *out = s.ptr;
+        MGX_HOST_CHECK(cudaHostAlloc(reinterpret_cast<void **>(&out->ptr), kParts * sizeof(val::ConstPart),
+                                     cudaHostAllocPortable | cudaHostAllocMapped));
+        out->ctx = ctx;
         return MGX_SUCCESS;
     }
+
+    void give_back(const Buffer &b)
+    {
+        if (b.ctx != 0) {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (count_ == kIdle && idle_[0].ctx != b.ctx) remove(0);  // of a context that may be gone
+            if (count_ < kIdle) {
+                idle_[count_++] = b;
+                return;
+            }
+        }
+        cudaFreeHost(b.ptr);
+    }
+
+    // Frees the idle buffers of the current context.
+    void trim()
+    {
+        const unsigned long long ctx = mgx_context_id();
+        Buffer mine[kIdle];
+        int n = 0;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            for (int i = count_ - 1; i >= 0; --i)
+                if (idle_[i].ctx == ctx) mine[n++] = remove(i);
+        }
+        while (n > 0) cudaFreeHost(mine[--n].ptr);
+    }
+
+private:
+    Buffer remove(int i)
+    {
+        const Buffer b = idle_[i];
+        for (--count_; i < count_; ++i) idle_[i] = idle_[i + 1];
+        return b;
+    }
+
+    std::mutex mu_;
+    Buffer idle_[kIdle];
+    int count_ = 0;
 };
 
+PartsPool &parts_pool()
+{
+    static PartsPool *pool = new PartsPool;
+    return *pool;
+}
+
 }  // namespace
+
+void mgx_validate_trim() { parts_pool().trim(); }
 
 int mgx_validate_impl(const double *d_c, size_t count, double expected, double abs_tol, double rel_tol,
                       mgx_validation_t *out, cudaStream_t stream)
@@ -270,10 +317,10 @@ int mgx_validate_impl(const double *d_c, size_t count, double expected, double a
     out->invalid = 0;
     out->max_abs_error = out->max_rel_error = 0.0;
     if (count > 0) {
-        static thread_local PartsBuffers buffers;
-        val::ConstPart *parts = nullptr;
-        const int brc = buffers.take(&parts);
+        PartsPool::Buffer buffer{};
+        const int brc = parts_pool().take(&buffer);
         if (brc != MGX_SUCCESS) return brc;
+        val::ConstPart *parts = buffer.ptr;
         size_t blocks = (count + 4 * val::THREADS - 1) / (4 * val::THREADS);  // four elements per step
         const size_t cap = (size_t)mgx_sm_count() * 8;
         if (blocks > cap) blocks = cap;
@@ -284,12 +331,13 @@ int mgx_validate_impl(const double *d_c, size_t count, double expected, double a
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) {
             mgx_set_last_cuda_error(e, "constant validation", __FILE__, __LINE__);
-            return MGX_E_CUDA;
+            return MGX_E_CUDA;  // (the buffer is not handed back: the kernel may still write to it)
         }
         for (size_t b = 0; b < blocks; ++b) {
             out->invalid += parts[b].invalid;
             if (parts[b].max_abs > out->max_abs_error) out->max_abs_error = parts[b].max_abs;
         }
+        parts_pool().give_back(buffer);
     }
     // an infinite `expected` gives NaN quotients, which never count
     const double rel = fabs(expected) > 0.0 ? out->max_abs_error / fabs(expected) : 0.0;
