@@ -12,7 +12,7 @@
 //   h = 0; for d = s+1 down to 2: h = fma(h, 2^-7, G_d);   C_ij (+)= h * 2^(ea_i + eb_j - 12).
 //
 // Kernels:
-//   ozaki_row_exp   row maxima of A (one block per row); clears the column statistics
+//   ozaki_row_exp   row maxima of A (a block, or a warp, per row); clears the column statistics
 //   ozaki_col_max   column maxima of B (atomicMax on the bit pattern of |b|); the last block of a
 //                   column group takes the exponents
 //   ozaki_split_a   digits of A as swizzled K-major tiles, blocked [row tile][K block][slice]
@@ -119,20 +119,24 @@ __global__ void __launch_bounds__(256) ozaki_zero(const ColStats z)
     zero_stats(z, blockIdx.x * 256 + threadIdx.x, gridDim.x * 256ll);
 }
 
-// One block of T threads per row, eight loads in flight per thread (with one warp per row, a short, wide
-// A occupied a few SMs: the split phase of 128 x 2000 x 16384 took 318 us, 149 now).
-template <int T>
-__global__ void __launch_bounds__(T) ozaki_row_exp(const double *__restrict__ A, int m, int k, int lda,
-                                                   int *__restrict__ ea, const ColStats z, int *status)
+// T threads per row, R rows per block (R > 1: a warp each), eight loads in flight per thread.  With one
+// warp per row for every k, a short, wide A occupied a few SMs: the split phase of 128 x 2000 x 16384 took
+// 318 us, 149 now.  With one row per block for every m, the blocks' starts took the time of a tall,
+// narrow A: 300000 x 64 x 64, 3 slices, 537 us, against 309 with eight.
+template <int T, int R>
+__global__ void __launch_bounds__(T * R) ozaki_row_exp(const double *__restrict__ A, int m, int k, int lda,
+                                                       int *__restrict__ ea, const ColStats z, int *status)
 {
+    static_assert(R == 1 || T == 32, "several rows: a warp each");
     __shared__ unsigned long long red[T / 32];
     pdl_wait();
     pdl_trigger();
-    zero_stats(z, (long long)blockIdx.x * T + threadIdx.x, (long long)gridDim.x * T);
-    const int row = blockIdx.x;
+    zero_stats(z, (long long)blockIdx.x * (T * R) + threadIdx.x, (long long)gridDim.x * (T * R));
+    const int row = blockIdx.x * R + threadIdx.x / T, tid = threadIdx.x % T;
+    if (R > 1 && row >= m) return;
     const unsigned long long *r = reinterpret_cast<const unsigned long long *>(A + (size_t)row * lda);
     unsigned long long mx = 0;
-    int kk = threadIdx.x;
+    int kk = tid;
     for (; kk + 7 * T < k; kk += 8 * T) {
         unsigned long long v[8];
 #pragma unroll
@@ -148,9 +152,11 @@ __global__ void __launch_bounds__(T) ozaki_row_exp(const double *__restrict__ A,
         const unsigned long long other = __shfl_xor_sync(0xffffffffu, mx, o);
         mx = other > mx ? other : mx;
     }
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    if (T > 32) {
+        if ((tid & 31) == 0) red[tid >> 5] = mx;
+        __syncthreads();
+    }
+    if (tid == 0) {
         for (int w = 1; w < T / 32; ++w) mx = red[w] > mx ? red[w] : mx;
         if (mx >= 0x7ff0000000000000ull) {
             ea[row] = NONFINITE_EXP;
@@ -781,13 +787,15 @@ static int ozaki_split_a_impl(const double *A, int m, int k, int lda, int s, uns
     int *status = mgx_device_status_ptr();
     int *ea = reinterpret_cast<int *>(ws + L.ea);
     const int kblocks = (k + 31) / 32;
-    // enough threads that a row is a few batches of loads
-    auto scan = [&](auto kernel, int threads) {
-        return mgx_launch_dependent(kernel, dim3((unsigned)m), dim3(threads), 0, stream, A, m, k, lda, ea, zero, status);
+    // enough threads that a row is a few batches of loads; rows share blocks where these still fill the SMs
+    auto scan = [&](auto kernel, int threads, int rows) {
+        return mgx_launch_dependent(kernel, dim3((unsigned)((m - 1) / rows + 1)), dim3(threads * rows), 0, stream, A, m, k,
+                                    lda, ea, zero, status);
     };
-    MGX_HOST_CHECK(k <= 512    ? scan(oz::ozaki_row_exp<32>, 32)
-                   : k <= 2048 ? scan(oz::ozaki_row_exp<128>, 128)
-                               : scan(oz::ozaki_row_exp<256>, 256));
+    MGX_HOST_CHECK(k <= 512 && m >= 8 * mgx_sm_count() ? scan(oz::ozaki_row_exp<32, 8>, 32, 8)
+                   : k <= 512                          ? scan(oz::ozaki_row_exp<32, 1>, 32, 1)
+                   : k <= 2048                         ? scan(oz::ozaki_row_exp<128, 1>, 128, 1)
+                                                       : scan(oz::ozaki_row_exp<256, 1>, 256, 1));
     return dispatch_splits<SplitA>(s, A, m, k, lda, kblocks, (const int *)ea, ws + L.da, stream);
 }
 
