@@ -627,32 +627,38 @@ __global__ void splitk_reduce(double *__restrict__ C, int ldc, int beta_one, con
 struct Pack {
     const double *src;
     double *dst;
-    int cols, live, ld_src;  // destination pitch (even), live columns, source pitch
-    int chunks;              // column chunks of a row
+    int rows, cols, live, ld_src;  // destination pitch (even), live columns, source pitch
+    int log2_width;                // threads of a row: 2^log2_width, each PACK_PER columns
+    int chunks;                    // column chunks of a row
+    unsigned blocks;
 };
 constexpr int PACK_THREADS = 256, PACK_PER = 8;
 
-// Both operands in one launch: block b < blocks_a packs one row chunk of A, the others B's.  Bound by
+// Both operands in one launch: blocks [0, a.blocks) pack A, the others B; a block packs one column chunk
+// of PACK_THREADS >> log2_width rows, the narrowest power of two of threads that a row's columns keep
+// busy (a block for each row however short: 2,000,000 rows of 3 took as many blocks).  Bound by
 // memory: 8-byte accesses because an odd pitch allows no wider ones, eight in flight per thread (a
 // grid-stride loop with a 64-bit division per element took 42 us for 98 MB, this takes 26).
-__global__ void __launch_bounds__(PACK_THREADS) pack_kernel(const Pack a, const Pack b, long long blocks_a)
+__global__ void __launch_bounds__(PACK_THREADS) pack_kernel(const Pack a, const Pack b)
 {
-    const bool is_a = blockIdx.x < blocks_a;
+    const bool is_a = blockIdx.x < a.blocks;
     const Pack &q = is_a ? a : b;
-    const long long i = is_a ? blockIdx.x : blockIdx.x - blocks_a;
-    const long long r = i / q.chunks;
-    const int c0 = (int)(i - r * q.chunks) * (PACK_THREADS * PACK_PER) + threadIdx.x;
+    const unsigned i = is_a ? blockIdx.x : blockIdx.x - a.blocks;
+    const int width = 1 << q.log2_width;
+    const long long r = (long long)(i / q.chunks) * (PACK_THREADS >> q.log2_width) + (threadIdx.x >> q.log2_width);
+    if (r >= q.rows) return;
+    const int c0 = (int)(i % q.chunks) * (width * PACK_PER) + (threadIdx.x & (width - 1));
     const double *src = q.src + r * q.ld_src;
     double *dst = q.dst + r * q.cols;
     double v[PACK_PER];
 #pragma unroll
     for (int u = 0; u < PACK_PER; ++u) {
-        const int c = c0 + u * PACK_THREADS;
+        const int c = c0 + u * width;
         v[u] = c < q.live ? __ldg(src + c) : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < PACK_PER; ++u) {
-        const int c = c0 + u * PACK_THREADS;
+        const int c = c0 + u * width;
         if (c < q.cols) dst[c] = v[u];
     }
 }
@@ -850,30 +856,33 @@ static int launch_dgemm(const double *A, const double *B, double *C, int m, int 
     const bool b_ok = ((reinterpret_cast<uintptr_t>(B) & 15) == 0) && ldb % 2 == 0;
     char *scratch = nullptr;
     if (!a_ok || !b_ok) {
-        const int chunk = fp64::PACK_THREADS * fp64::PACK_PER;
         const int lda2 = (k_len + 1) & ~1, ldb2 = (n + 1) & ~1;
         const size_t abytes = a_ok ? 0 : ((size_t)m * lda2 * sizeof(double) + 255) & ~size_t(255);
         const size_t bbytes = b_ok ? 0 : (size_t)b_rows * ldb2 * sizeof(double);
         const int arc = mgx_scratch_alloc(reinterpret_cast<void **>(&scratch), abytes + bbytes + 256, stream);
         if (arc != MGX_SUCCESS) return arc;
+        auto pack = [](const double *src, char *dst, int rows, int cols, int live, int ld) {
+            fp64::Pack q = {src, reinterpret_cast<double *>(dst), rows, cols, live, ld, 0, 0, 0u};
+            while ((fp64::PACK_PER << q.log2_width) < cols && (1 << q.log2_width) < fp64::PACK_THREADS) ++q.log2_width;
+            const int chunk = fp64::PACK_PER << q.log2_width, per = fp64::PACK_THREADS >> q.log2_width;
+            q.chunks = (cols - 1) / chunk + 1;
+            q.blocks = (unsigned)((rows - 1) / per + 1) * (unsigned)q.chunks;
+            return q;
+        };
         fp64::Pack qa = {}, qb = {};
-        long long blocks_a = 0, blocks_b = 0;
-        qa.chunks = qb.chunks = 1;
         if (!a_ok) {
-            qa = {A + a_x0, reinterpret_cast<double *>(scratch), lda2, a_x_end - a_x0, lda, (lda2 + chunk - 1) / chunk};
-            blocks_a = (long long)m * qa.chunks;
+            qa = pack(A + a_x0, scratch, m, lda2, a_x_end - a_x0, lda);
             A = qa.dst;
             lda = lda2;
             a_x0 = 0;
             a_x_end = k_len;
         }
         if (!b_ok) {
-            qb = {B, reinterpret_cast<double *>(scratch + abytes), ldb2, n, ldb, (ldb2 + chunk - 1) / chunk};
-            blocks_b = (long long)b_rows * qb.chunks;
+            qb = pack(B, scratch + abytes, b_rows, ldb2, n, ldb);
             B = qb.dst;
             ldb = ldb2;
         }
-        fp64::pack_kernel<<<(unsigned)(blocks_a + blocks_b), fp64::PACK_THREADS, 0, stream>>>(qa, qb, blocks_a);
+        fp64::pack_kernel<<<qa.blocks + qb.blocks, fp64::PACK_THREADS, 0, stream>>>(qa, qb);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
             mgx_set_last_cuda_error(e, "operand packing", __FILE__, __LINE__);
