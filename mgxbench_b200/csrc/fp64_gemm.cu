@@ -78,7 +78,7 @@ struct Params {
     int m, n;
     int a_x0;         // first column of A (k_offset)
     int ldc;
-    int beta_one;
+    int beta_one;     // 1: C + A B, 0: A B, -1: 0 + A B (no negative zeros)
     int vec_store;    // C rows 16-byte aligned (ldc even, C aligned)
     int *status;
     int bands, ucols;   // ceil(m / BM), ceil(n / 8)
@@ -441,14 +441,15 @@ __global__ void __launch_bounds__(THREADS, 1)
                 if (vec_store && col + 1 < p.n) {
                     double2 *dst = reinterpret_cast<double2 *>(crow + col);
                     if (beta_one) {
-                        const double2 old = *dst;
+                        double2 old = make_double2(0.0, 0.0);
+                        if (beta_one > 0) old = *dst;
                         v0 = old.x + v0;
                         v1 = old.y + v1;
                     }
                     *dst = make_double2(v0, v1);
                 } else {
-                    crow[col] = beta_one ? crow[col] + v0 : v0;
-                    if (col + 1 < p.n) crow[col + 1] = beta_one ? crow[col + 1] + v1 : v1;
+                    crow[col] = beta_one ? (beta_one > 0 ? crow[col] : 0.0) + v0 : v0;
+                    if (col + 1 < p.n) crow[col + 1] = beta_one ? (beta_one > 0 ? crow[col + 1] : 0.0) + v1 : v1;
                 }
             }
         }
@@ -751,7 +752,7 @@ static int launch_dgemm(const double *A, const double *B, double *C, int m, int 
 {
     if (m <= 0 || n <= 0) return MGX_SUCCESS;
     if (k_len <= 0) {
-        if (beta_one) return MGX_SUCCESS;
+        if (beta_one > 0) return MGX_SUCCESS;
         // C = A*B with an empty reduction is zero
         MGX_HOST_CHECK(cudaMemset2DAsync(C, (size_t)ldc * sizeof(double), 0, (size_t)n * sizeof(double), m, stream));
         return MGX_SUCCESS;
@@ -924,21 +925,22 @@ static int launch_dgemm(const double *A, const double *B, double *C, int m, int 
 }
 
 // C (+)= A[:, a_x0 : a_x0 + k_len] * B[0 : k_len, :] with the library's FP64 kernel.
-// a_x_end: A columns at or beyond it read as zero; b_rows: rows of B that exist.
+// a_x_end: A columns at or beyond it read as zero; b_rows: rows of B that exist.  beta_one: 1 adds to C, 0
+// writes the product, -1 writes 0 + the product (the first of several panels).
 int mgx_launch_dgemm(const double *A, const double *B, double *C, int m, int n, int k_len, int a_x0, int a_x_end,
                      int b_rows, int lda, int ldb, int ldc, int beta_one, cudaStream_t stream)
 {
     return launch_dgemm(A, B, C, m, n, k_len, a_x0, a_x_end, b_rows, lda, ldb, ldc, beta_one, stream, DgemmMode{});
 }
 
-// SUMMA: C = sum over the panels of width panel_k (a multiple of 32) of A B, each panel's product
-// added with one rounding.
+// SUMMA: C = 0 + the sum over the panels of width panel_k (a multiple of 32, or all of K) of A B, each
+// panel's product added with one rounding.
 int mgx_launch_dgemm_panels(const double *A, const double *B, double *C, int m, int n, int k, int lda, int ldb,
                             int ldc, int panel_k, cudaStream_t stream)
 {
     DgemmMode mode;
     mode.panel_k = panel_k;
-    return launch_dgemm(A, B, C, m, n, k, 0, k, k, lda, ldb, ldc, 0, stream, mode);
+    return launch_dgemm(A, B, C, m, n, k, 0, k, k, lda, ldb, ldc, -1, stream, mode);
 }
 
 // Split-K form: the K range is cut into `ksplit` slices whose products land in `partial`

@@ -157,8 +157,8 @@ MGX_API int mgx_summa_run(mgx_summa_plan_t *P, const double *A, int lda, const d
     // of which writes C (0 + its product).
     for (int k0 = 0; k0 < d.k; k0 += d.panel_k) {
         const int kc = (d.k - k0 < d.panel_k) ? d.k - k0 : d.panel_k;
-        const int rc = mgx_launch_dgemm(A, B + (size_t)k0 * ldb, C, d.m, d.n, kc, k0, k0 + kc, kc, lda, ldb, ldc, k0 > 0,
-                                        s);
+        const int rc = mgx_launch_dgemm(A, B + (size_t)k0 * ldb, C, d.m, d.n, kc, k0, k0 + kc, kc, lda, ldb, ldc,
+                                        k0 > 0 ? 1 : -1, s);
         if (rc != MGX_SUCCESS) return rc;
     }
     return MGX_SUCCESS;
