@@ -29,6 +29,7 @@
 // An element's reduction runs over K in the same order whatever the tile width or the share it falls
 // in, so the cut does not change a bit of the result.
 #include <atomic>
+#include <chrono>
 #include <cstdio>
 #include <cstring>
 #include <type_traits>
@@ -738,6 +739,23 @@ size_t mgx_fp64_streamk_bytes(int m, int n, int k)
            ((tiles * fp64::CWARPS * sizeof(unsigned long long) + 255) & ~size_t(255));
 }
 
+// A fresh ticket tag per stream-K launch, 56 bits.  Odd, so that cleared memory reads as no arrivals, and
+// counted from a start that differs from process to process: the workspace is the caller's, never cleared,
+// and small tags would be found in what other programs leave in memory, such as an array of indices.
+static unsigned long long streamk_tag()
+{
+    static std::atomic<unsigned long long> next{[] {
+        // splitmix64 (Steele, Lea and Flood 2014) of the time and of an address of this process
+        unsigned long long z = (unsigned long long)std::chrono::high_resolution_clock::now().time_since_epoch().count();
+        z ^= (unsigned long long)reinterpret_cast<uintptr_t>(&z) << 20;
+        z += 0x9e3779b97f4a7c15ull;
+        z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+        z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+        return z ^ (z >> 31);
+    }()};
+    return (next.fetch_add(2, std::memory_order_relaxed) | 1ull) & ((1ull << 56) - 1);
+}
+
 // How launch_dgemm cuts and accumulates a product (the defaults: one whole-K product).
 struct DgemmMode {
     int panel_k = 0;   // > 0: SUMMA panels of this width, a multiple of 32
@@ -839,9 +857,7 @@ static int launch_dgemm(const double *A, const double *B, double *C, int m, int 
         }
         p.sk_partial = reinterpret_cast<double *>(mode.ws);
         p.sk_tickets = reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(mode.ws) + pbytes);
-        // a fresh tag per launch (56 bits, never 0: zeroed memory reads as no arrivals)
-        static std::atomic<unsigned long long> epochs{0};
-        p.sk_epoch = ((epochs.fetch_add(1, std::memory_order_relaxed) + 1) & ((1ull << 56) - 1));
+        p.sk_epoch = streamk_tag();
     }
 
     // TMA wants 16-byte aligned bases, pitches and (even) columns; operands that are not so are
