@@ -43,7 +43,9 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
+#include "crt_pairs.h"
 #include "mgx_common.cuh"
 
 namespace mgx {
@@ -1417,6 +1419,50 @@ CrtView crt_view(const CrtLayout &L, unsigned char *ws, int r0, int c0, int m, i
     return v;
 }
 
+// Pairs of CTAs that the current context's SMs hold at once: one per two SMs on a whole B200, fewer where a
+// partition has SMs without a partner.  More clusters than that would start only when others have ended, and
+// every item of those would wait out the lockstep's limit for them.  Asked once per context (its id is
+// never used again); without an id, each time.  0 (CTAs alone) where it cannot be told.
+int crt_pair_slots()
+{
+    struct Known {
+        unsigned long long ctx;
+        int clusters;
+    };
+    static std::mutex mu;
+    static Known known[64];
+    static int count = 0;
+    const unsigned long long ctx = mgx_context_id();
+    if (ctx != 0) {
+        std::lock_guard<std::mutex> lk(mu);
+        for (int i = 0; i < count; ++i)
+            if (known[i].ctx == ctx) return known[i].clusters;
+    }
+    constexpr int smem = crt::Ring<true>::SMEM_BYTES;
+    const int most = mgx_sm_count() / 2;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2u * (unsigned)(most > 0 ? most : 1));
+    cfg.blockDim = dim3(crt::THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int active = 0;
+    if (cudaFuncSetAttribute(crt::crt_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&active, crt::crt_gemm<true>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (ctx != 0) {
+        std::lock_guard<std::mutex> lk(mu);
+        if (count < 64) known[count++] = Known{ctx, active};
+    }
+    return active;
+}
+
 // Residue products of a block on the tensor cores (one persistent launch).
 int crt_products_impl(const crt::Consts &K, const CrtLayout &L, const CrtView &v, cudaStream_t stream,
                       unsigned int *sync = nullptr)
@@ -1458,11 +1504,10 @@ int crt_products_impl(const crt::Consts &K, const CrtLayout &L, const CrtView &v
         MGX_HOST_CHECK(cudaMemsetAsync(sync, 0, sizeof(unsigned int), stream));
         p.sync = sync;
     }
-    // CTA pairs where their rounds of items are no more than single CTAs' (an odd last tile row makes
-    // half a pair idle) and four rounds or more pay for the pairs' setup: 1333 x 2011 x 1777, 5 rounds,
-    // 143 us against 147 alone; 1024^3, 2 rounds, 62.9 against 62.5.
-    const long long pairs = (long long)K.q * ((v.tiles_m + 1) / 2) * v.tiles_n * L.ksplit, slots = sms / 2;
-    if (slots > 0 && pairs >= 4 * slots && (pairs + slots - 1) / slots <= (items + sms - 1) / sms) {
+    const long long pairs = (long long)K.q * ((v.tiles_m + 1) / 2) * v.tiles_n * L.ksplit;
+    int slots = crt::pairs_to_launch(items, pairs, sms, sms / 2);
+    if (slots > 0) slots = crt::pairs_to_launch(items, pairs, sms, crt_pair_slots());
+    if (slots > 0) {
         int rc = mgx_encode_tmap_3d(&p.ma, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, v.ra, 256, 8, K.q * p.a_slabs - v.a_slab0,
                                     1024, crt::SLAB, 256, 8, crt::KPACK, CU_TENSOR_MAP_SWIZZLE_NONE);
         if (rc == MGX_SUCCESS)
