@@ -34,16 +34,12 @@
 #include <cstring>
 #include <type_traits>
 
+#include "fp64_cut.h"
 #include "mgx_common.cuh"
 
 namespace mgx {
 namespace fp64 {
 
-constexpr int BK = 32;
-constexpr int UNIT = 8;                                   // columns of a work unit (one DMMA's N)
-constexpr int TILE_UNITS = 16;                            // widest tile: 128 columns
-constexpr int BM = 64;                                    // rows of a band
-constexpr int CWARPS = 16;
 constexpr int SUB_WARPS = CWARPS / 4;                     // consumer warps of a sub-partition
 constexpr int WARP_UNITS = (TILE_UNITS + SUB_WARPS - 1) / SUB_WARPS;  // units of a consumer warp
 constexpr int PRODUCER_WARPS = 4;                         // one warpgroup
@@ -65,16 +61,8 @@ constexpr int A_STAGE_BYTES = 2 * A_BOX_BYTES;
 constexpr int STAGE_BYTES = A_STAGE_BYTES + 8 * B_BOX_BYTES;
 constexpr int STAGES = 4;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
-constexpr int GROUP_M = 1024 / BM;           // stream-K raster groups of 1024 rows
-// A last band of at most 16 or 32 rows computes one or two 16-row strips, spread over all four
-// sub-partitions.  Its units then cost less by this measure, against COST for a whole band's; more than
-// a quarter and a half of it, because a warp has fewer units to hide its loads behind.  Sizes measured
-// with 2 and 4, 3 and 5, 4 and 6 of 8: 1040 x 4096 x 4096 1459, 991, 1008 us (1043 with whole bands
-// only), 1056 x 2048 x 4096 602, 505, 521 (526), 80 x 4096 x 4096 144, 128, 120 (143).  One band alone,
-// 8192 x 8192: 16 rows 279 -> 104 us, 32 rows 279 -> 189.
-constexpr int COST = 8, COST_1 = 3, COST_2 = 5;
 
-struct Params {
+struct Params : Cut {
     double *C;
     int m, n;
     int a_x0;         // first column of A (k_offset)
@@ -82,150 +70,14 @@ struct Params {
     int beta_one;     // 1: C + A B, 0: A B, -1: 0 + A B (no negative zeros)
     int vec_store;    // C rows 16-byte aligned (ldc even, C aligned)
     int *status;
-    int bands, ucols;   // ceil(m / BM), ceil(n / 8)
-    int tile_units;     // units of a whole tile (the last tile of a band may have fewer)
-    int tiles_n;        // ceil(ucols / tile_units)
-    int kblocks;        // K blocks of the whole reduction
-    int skew;           // units that starting another band costs a CTA (see Walk)
-    int strips_last;    // log2 of the 16-row strips of the last band that are computed: 0, 1 or 2
-    int w_full, w_last; // what a unit of a band, and of the last band, costs (see Walk)
-    long long length;   // the product's length by that measure, and its part per CTA
-    long long share;
-    int share_rem;      // length - share x grid
-    long long sk_full;  // stream-K: K-block units of the tiles that cost w_full
     int panel_kb;       // > 0: SUMMA panels of so many K blocks; the running sum takes each panel's product
                         // with one rounding
     unsigned long long *sk_tickets;  // stream-K: one arrival ticket per tile and consumer warp
     unsigned long long sk_epoch;     // stream-K: this launch's ticket tag (a ticket of another tag counts 0)
     double *sk_partial; // stream-K: two partial accumulators per CTA (its first and last segment)
-    int ksplit;         // K slices (1: whole K); slice s reduces K blocks [s kb_split, (s + 1) kb_split)
-    int kb_split;
     double *partial;    // split-K: slice s of the product goes to partial + s * partial_stride
     int partial_ld;     // even, so the partial rows are 16-byte aligned
     size_t partial_stride;
-};
-
-// One piece of work: units [u0, u0 + units) of a band over K blocks [kb_begin, kb_end).
-struct Item {
-    int band, u0, units, kb_begin, kb_end, slice;
-    int strips;  // log2 of the 16-row strips that are computed
-    int tile;    // stream-K: the tile this is a piece of
-};
-
-// Tile coordinates of raster position `tile`: groups of 1024 rows sweep the columns together; the
-// tiles of a last band that costs less come after all others.
-__device__ __forceinline__ void tile_coords(const Params &p, int tile, int &tm, int &tn)
-{
-    const int bands = p.w_last < p.w_full ? p.bands - 1 : p.bands;
-    if (tile >= bands * p.tiles_n) {
-        tm = bands;
-        tn = tile - bands * p.tiles_n;
-        return;
-    }
-    const int per_group = GROUP_M * p.tiles_n;
-    const int group = tile / per_group;
-    const int first_m = group * GROUP_M;
-    const int gsize = min(bands - first_m, GROUP_M);
-    const int r = tile % per_group;
-    tm = first_m + r % gsize;
-    tn = r / gsize;
-}
-
-// c U / G, where CTA c's share of a length U begins (U = share x G + share_rem).
-__device__ __forceinline__ long long sk_begin(const Params &p, unsigned c)
-{
-    return c * p.share + c * (unsigned)p.share_rem / gridDim.x;
-}
-
-// CTA whose share holds unit u (sk_begin(c) <= u < sk_begin(c + 1)).
-__device__ __forceinline__ int sk_owner(long long u, long long U, long long G)
-{
-    return (int)(((u + 1) * G + U - 1) / U - 1);
-}
-
-// Stream-K units are the K blocks of the tiles, in raster order.  They cost w_full each, those of a last
-// band of one or two strips w_last; where a unit starts on that scale, and the whole product's length.
-__device__ __forceinline__ long long sk_start(const Params &p, long long x)
-{
-    return x < p.sk_full ? x * p.w_full : p.sk_full * p.w_full + (x - p.sk_full) * p.w_last;
-}
-// The first unit that starts at `pos` or later.
-__device__ __forceinline__ long long sk_unit(const Params &p, long long pos)
-{
-    const long long rest = pos - p.sk_full * p.w_full;
-    if (p.w_full == 1) return pos;
-    return rest <= 0 ? (pos + p.w_full - 1) / p.w_full : p.sk_full + (rest + p.w_last - 1) / p.w_last;
-}
-
-// The work of one CTA, shared by the producer and the consumers: the units that start in its equal
-// share of the product's length.
-//   Regular: the units of all (band, K slice) rows, in that order, cut into pieces no wider than a
-//   tile.  A share that runs on into another band works on two narrower pieces, which load A
-//   twice and leave some warps without a unit, so each row is given `skew` virtual units at its
-//   start that carry no work.
-//   Stream-K: the pieces of consecutive tiles' K ranges.
-template <bool STREAMK, typename Unit>
-struct Walk {
-    Unit x, x_end;  // the share's next unit and its end
-
-    // (32 bits hold every position: a row's length is at most its part of C's bytes / 512)
-    static __device__ __forceinline__ unsigned row_unit(const Params &p, unsigned pos)
-    {
-        const unsigned len = (p.ucols + p.skew) * p.w_full, head = p.skew * p.w_full;
-        unsigned slice = 0;
-        if (p.ksplit > 1) {
-            const unsigned slice_len = (unsigned)p.length / (unsigned)p.ksplit;
-            slice = pos / slice_len;
-            pos -= slice * slice_len;
-        }
-        const unsigned band = min(pos / len, (unsigned)p.bands - 1u), off = pos - band * len;
-        const unsigned w = band == p.bands - 1u ? p.w_last : p.w_full;
-        unsigned first = off <= head ? 0u : off - head;
-        if (w > 1) first = (first + w - 1) / w;
-        return (slice * p.bands + band) * p.ucols + first;
-    }
-
-    __device__ __forceinline__ void init(const Params &p)
-    {
-        const long long begin = sk_begin(p, blockIdx.x), end = sk_begin(p, blockIdx.x + 1);
-        if constexpr (STREAMK) {
-            x = sk_unit(p, begin);
-            x_end = sk_unit(p, end);
-        } else {
-            x = row_unit(p, (unsigned)begin);
-            x_end = row_unit(p, (unsigned)end);
-        }
-    }
-
-    __device__ __forceinline__ bool next(const Params &p, Item &it)
-    {
-        if (x >= x_end) return false;
-        if constexpr (STREAMK) {
-            it.tile = (int)(x / p.kblocks);
-            int tn;
-            tile_coords(p, it.tile, it.band, tn);
-            it.u0 = tn * p.tile_units;
-            it.units = min(p.tile_units, p.ucols - it.u0);
-            it.slice = 0;
-            it.kb_begin = (int)(x - (long long)it.tile * p.kblocks);
-            it.kb_end = (int)min((long long)p.kblocks, it.kb_begin + x_end - x);
-            x += it.kb_end - it.kb_begin;
-        } else {
-            const unsigned row = x / (unsigned)p.ucols;
-            const int off = (int)(x - row * p.ucols);
-            const int run = min(p.ucols - off, (int)(x_end - x));  // the row's units in this share
-            const int pieces = (run + TILE_UNITS - 1) / TILE_UNITS;
-            it.slice = p.ksplit > 1 ? row / p.bands : 0;
-            it.band = row - it.slice * p.bands;
-            it.u0 = off;
-            it.units = (run + pieces - 1) / pieces;
-            it.kb_begin = it.slice * p.kb_split;
-            it.kb_end = min(p.kblocks, it.kb_begin + p.kb_split);
-            x += it.units;
-        }
-        it.strips = it.band == p.bands - 1 ? p.strips_last : 2;
-        return true;
-    }
 };
 
 // Stream-K tickets: (launch tag << 8) | arrivals.  A ticket written by an earlier launch (another
@@ -372,7 +224,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     // live: 3001 x 5002 x 4096 in panels of 512 takes 3496 us with 64-bit positions, 3565 with 32-bit
     // ones.  The whole-K form is 1.5% faster with 32-bit ones at N = 256.
     Walk<STREAMK, std::conditional_t<PANELS || STREAMK, long long, unsigned>> walk;
-    walk.init(p);
+    walk.init(p, blockIdx.x, gridDim.x);
     Item it;
 
     if (warp < PRODUCER_WARPS) {
@@ -457,14 +309,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     };
 
     while (walk.next(p, it)) {
-        // This warp's strip and part of the tile's units.  Warps cw, cw + 4, ... share a sub-partition:
-        // its 16 rows of a whole band, so an uneven split of the units does not unbalance anything.
-        // One or two strips are spread over all sub-partitions, a column's units over neighbours.
-        if (PANELS) it.strips = 2;  // (a variable one costs 1%; the host asks for no other)
-        c.strip = cw & ((1 << it.strips) - 1);
-        const int sharers = CWARPS >> it.strips, per = (it.units + sharers - 1) >> (4 - it.strips);
-        c.u_first = (cw >> it.strips) * per;
-        const int nu = max(0, min(per, it.units - c.u_first));
+        if (PANELS) it.strips = 2;  // (a variable one costs 1%; make_cut asks for no other)
+        int nu;
+        warp_part(it, cw, c.strip, c.u_first, nu);
 
         double acc[WARP_UNITS][4];
         double tot[PANELS ? WARP_UNITS : 1][4];
@@ -497,10 +344,8 @@ __global__ void __launch_bounds__(THREADS, 1)
             // arrives last at its ticket: every piece's accumulator goes to that CTA's partial
             // slot, and the last arrival adds the pieces in K order (p0 + p1) + p2 ... and
             // stores C.  No CTA waits for another.
-            const long long U = p.length, NG = gridDim.x;
-            const long long t0 = (long long)it.tile * p.kblocks;
-            const int c0 = sk_owner(sk_start(p, t0), U, NG);
-            const int pieces = sk_owner(sk_start(p, t0 + p.kblocks - 1), U, NG) - c0 + 1;
+            const Piece q = piece_of(p, it, blockIdx.x, gridDim.x);
+            const int pieces = q.pieces, j = q.index;
             if (pieces == 1) {
                 store_acc(acc, nu, p.beta_one, p.C, p.ldc, p.vec_store);
             } else {
@@ -510,8 +355,6 @@ __global__ void __launch_bounds__(THREADS, 1)
                 constexpr int NACC = WARP_UNITS * 4;
                 constexpr size_t PART = (size_t)CWARPS * 32 * NACC;  // doubles per partial slot
                 const int ct = threadIdx.x - PRODUCER_WARPS * 32;     // consumer thread 0..511
-                const int j = (int)blockIdx.x - c0;                    // this CTA's piece
-                const int slot = (t0 + it.kb_begin == sk_unit(p, sk_begin(p, blockIdx.x))) ? 0 : 1;
                 double(&af)[NACC] = reinterpret_cast<double(&)[NACC]>(acc);
                 const int na = nu * 4;
                 unsigned long long *ticket = p.sk_tickets + (size_t)it.tile * CWARPS + cw;
@@ -524,7 +367,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     last = __shfl_sync(0xffffffffu, last, 0);
                 }
                 if (!last) {
-                    double *mine = p.sk_partial + ((size_t)blockIdx.x * 2 + slot) * PART;
+                    double *mine = p.sk_partial + ((size_t)blockIdx.x * 2 + q.slot) * PART;
 #pragma unroll
                     for (int i = 0; i < NACC; ++i)
                         if (i < na) __stcg(mine + (size_t)i * (CWARPS * 32) + ct, af[i]);
@@ -540,29 +383,28 @@ __global__ void __launch_bounds__(THREADS, 1)
                     // own piece (which has been written too, unless it is the first and never left its
                     // registers), 128 x 128 x 4096 with 74 pieces took 335 us, 83 now, 256^3 with 8 35 and 15.
                     constexpr int TRIP = 4;
-                    const int slot0 = (sk_unit(p, sk_begin(p, c0)) == t0) ? 0 : 1;
 #pragma unroll
                     for (int i0 = 0; i0 < NACC; i0 += 8) {
                         if (i0 >= na) break;
                         if (j > 0) {
-                            const double *p0 = p.sk_partial + ((size_t)c0 * 2 + slot0) * PART + ct;
+                            const double *p0 = p.sk_partial + ((size_t)q.c0 * 2 + q.slot0) * PART + ct;
 #pragma unroll
                             for (int i = 0; i < 8; ++i) af[i0 + i] = __ldcg(p0 + (i0 + i) * (CWARPS * 32));
                         }
                         for (int jj = 1; jj < pieces; jj += TRIP) {
                             double v[TRIP][8];
 #pragma unroll
-                            for (int q = 0; q < TRIP; ++q) {
+                            for (int r = 0; r < TRIP; ++r) {
                                 // pieces after the first start their CTA's share: slot 0
-                                const double *pq = p.sk_partial + (size_t)(c0 + min(jj + q, pieces - 1)) * 2 * PART + ct;
+                                const double *pr = p.sk_partial + (size_t)(q.c0 + min(jj + r, pieces - 1)) * 2 * PART + ct;
 #pragma unroll
-                                for (int i = 0; i < 8; ++i) v[q][i] = __ldcg(pq + (i0 + i) * (CWARPS * 32));
+                                for (int i = 0; i < 8; ++i) v[r][i] = __ldcg(pr + (i0 + i) * (CWARPS * 32));
                             }
 #pragma unroll
-                            for (int q = 0; q < TRIP; ++q)
-                                if (jj + q < pieces) {
+                            for (int r = 0; r < TRIP; ++r)
+                                if (jj + r < pieces) {
 #pragma unroll
-                                    for (int i = 0; i < 8; ++i) af[i0 + i] = af[i0 + i] + v[q][i];
+                                    for (int i = 0; i < 8; ++i) af[i0 + i] = af[i0 + i] + v[r][i];
                                 }
                         }
                     }
@@ -700,42 +542,19 @@ size_t mgx_fp64_splitk_bytes(int m, int n, int k, int ksplit)
     return (size_t)slices * (size_t)m * (size_t)((n + 1) & ~1) * sizeof(double) + 256;
 }
 
-// Bands, units and stream-K tiles of a product (tiles as even in width as the units allow, so a
-// ragged last tile wastes little: 1281 columns are eleven tiles of 15 units, not ten of 16 and one).
-struct DgemmCut {
-    int bands, ucols, tile_units, tiles_n;
-};
-
-static DgemmCut dgemm_cut(int m, int n)
-{
-    DgemmCut c;
-    c.bands = (m + fp64::BM - 1) / fp64::BM;
-    c.ucols = (n + fp64::UNIT - 1) / fp64::UNIT;
-    c.tiles_n = (c.ucols + fp64::TILE_UNITS - 1) / fp64::TILE_UNITS;
-    c.tile_units = (c.ucols + c.tiles_n - 1) / c.tiles_n;
-    return c;
-}
-
 // Stream-K workspace: two partial accumulators (64 x 128 doubles) per CTA of the grid, then one 8-byte
 // ticket per tile and consumer warp.
 static size_t streamk_partial_bytes(int grid)
 {
     return (size_t)grid * 2 * fp64::CWARPS * 32 * fp64::WARP_UNITS * 4 * sizeof(double);
 }
-static int streamk_grid(int m, int n, int k)
-{
-    const DgemmCut c = dgemm_cut(m, n);
-    const long long units = (long long)c.bands * c.tiles_n * ((k + fp64::BK - 1) / fp64::BK);
-    const int sms = mgx_sm_count();
-    return units < sms ? (int)units : sms;
-}
 
 size_t mgx_fp64_streamk_bytes(int m, int n, int k)
 {
     if (m <= 0 || n <= 0 || k <= 0) return 0;
-    const DgemmCut c = dgemm_cut(m, n);
+    const fp64::Cut c = fp64::shape_cut(m, n, k);
     const size_t tiles = (size_t)c.bands * c.tiles_n;
-    return streamk_partial_bytes(streamk_grid(m, n, k)) +
+    return streamk_partial_bytes(fp64::streamk_grid(c, mgx_sm_count())) +
            ((tiles * fp64::CWARPS * sizeof(unsigned long long) + 255) & ~size_t(255));
 }
 
@@ -775,8 +594,17 @@ static int launch_dgemm(const double *A, const double *B, double *C, int m, int 
         MGX_HOST_CHECK(cudaMemset2DAsync(C, (size_t)ldc * sizeof(double), 0, (size_t)n * sizeof(double), m, stream));
         return MGX_SUCCESS;
     }
+    const bool panels = mode.panel_k > 0 && mode.panel_k < k_len;
+    int slices = 1, kb_split = 0, grid = 0;
+    splitk_geometry(k_len, panels ? 1 : mode.ksplit, &kb_split, &slices);
     fp64::Params p;
     memset(&p, 0, sizeof p);
+    static_cast<fp64::Cut &>(p) =
+        fp64::make_cut(m, n, k_len, slices, kb_split,
+                       panels         ? fp64::CutMode::kPanels
+                       : mode.streamk ? fp64::CutMode::kStreamK
+                                      : fp64::CutMode::kWhole,
+                       mgx_sm_count(), &grid);
     p.C = C;
     p.m = m;
     p.n = n;
@@ -784,11 +612,6 @@ static int launch_dgemm(const double *A, const double *B, double *C, int m, int 
     p.beta_one = beta_one;
     p.vec_store = ((ldc & 1) == 0) && ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
     p.status = mgx_device_status_ptr();
-    const bool panels = mode.panel_k > 0 && mode.panel_k < k_len;
-    int slices = 1;
-    splitk_geometry(k_len, panels ? 1 : mode.ksplit, &p.kb_split, &slices);
-    p.ksplit = slices;
-    p.kblocks = (k_len + fp64::BK - 1) / fp64::BK;
     if (panels) p.panel_kb = mode.panel_k / fp64::BK;
     p.partial_ld = (n + 1) & ~1;
     p.partial_stride = (size_t)m * (size_t)p.partial_ld;
@@ -802,54 +625,13 @@ static int launch_dgemm(const double *A, const double *B, double *C, int m, int 
         p.partial = reinterpret_cast<double *>(mode.ws);
     }
 
-    const int sms = mgx_sm_count();
-    const DgemmCut cut = dgemm_cut(m, n);
-    p.bands = cut.bands;
-    p.ucols = cut.ucols;
-    p.tile_units = cut.tile_units;
-    p.tiles_n = cut.tiles_n;
-    const long long units = (long long)cut.bands * cut.ucols * slices;
-    int grid = units < sms ? (int)units : sms;
-    // A band crossing costs a CTA about two units of time (777 x 1282 x 6000: 419 us without, 404 with
-    // one and 388 with two virtual units; N = 1024 75.3, 70.8, 69.1).  With shares of a few units the
-    // virtual ones would take whole shares away, so they are left out there.
-    p.skew = units >= 8ll * grid ? 2 : 0;
-    if (mode.streamk) grid = streamk_grid(m, n, k_len);
-    // A last band of one or two strips (not in the panel form, see its kernel).  Stream-K: a CTA without
-    // a unit would be counted among a tile's pieces, so shares are no shorter than the longest unit.
-    // Where every CTA has one unit at most the weights would only move units together: 80 x 512 x 1024
-    // 13.0 us without them, 13.6 with.
-    p.strips_last = 2;
-    p.w_full = p.w_last = 1;
-    const int strips = (m - (cut.bands - 1) * fp64::BM + 15) / 16;
-    if (strips <= 2 && !panels) {
-        const int w = strips == 1 ? fp64::COST_1 : fp64::COST_2;
-        const long long row = (long long)cut.tiles_n * p.kblocks;
-        const bool weigh = cut.bands == 1 ? false
-                           : mode.streamk ? row * ((cut.bands - 1) * fp64::COST + w) >= (long long)grid * fp64::COST
-                                          : units > sms;
-        if (weigh) {
-            p.w_full = fp64::COST;
-            p.w_last = w;
-        }
-        if (weigh || cut.bands == 1 || !mode.streamk) p.strips_last = strips - 1;
-    }
-    if (mode.streamk) {
-        p.sk_full = (long long)(p.w_last < p.w_full ? cut.bands - 1 : cut.bands) * cut.tiles_n * p.kblocks;
-        p.length = p.sk_full * p.w_full + ((long long)cut.bands * cut.tiles_n * p.kblocks - p.sk_full) * p.w_last;
-    } else {
-        p.length = slices * ((cut.bands - 1) * (long long)(cut.ucols + p.skew) * p.w_full + p.skew * p.w_full +
-                             (long long)cut.ucols * p.w_last);
-    }
-    p.share = p.length / grid;
-    p.share_rem = (int)(p.length - p.share * grid);
     if (mode.streamk) {
         if (grid > 255) {  // arrivals per tile must fit a ticket's 8-bit count
             mgx_set_last_message("FP64 stream-K: grid of %d CTAs exceeds 255", grid);
             return MGX_E_UNSUPPORTED;
         }
         const size_t pbytes = streamk_partial_bytes(grid);
-        const size_t tbytes = (size_t)cut.bands * cut.tiles_n * fp64::CWARPS * sizeof(unsigned long long);
+        const size_t tbytes = (size_t)p.bands * p.tiles_n * fp64::CWARPS * sizeof(unsigned long long);
         if (!mode.ws || mode.ws_bytes < pbytes + tbytes || (reinterpret_cast<uintptr_t>(mode.ws) & 255)) {
             mgx_set_last_message("FP64 stream-K: workspace of %zu bytes (aligned to 256) needed, %zu given",
                                  pbytes + tbytes, mode.ws_bytes);
