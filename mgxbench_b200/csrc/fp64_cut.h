@@ -243,6 +243,9 @@ inline Cut make_cut(int m, int n, int k, int ksplit, int kb_split, CutMode mode,
     p.skew = units >= 8ll * *grid ? 2 : 0;
     // A last band of one or two strips (not in the panel form, see its kernel).  Stream-K: a CTA without
     // a unit would be counted among a tile's pieces, so shares are no shorter than the longest unit.
+    // Weighed only from shares of four whole units on: below that the weights make more pieces of the other
+    // tiles, whose sums cost more than the balance gives (71 x 201 x 2587, 2 units, 53.8 us with weights, 38.5
+    // without; 400^3, 2, 20.6 and 18.3; 65 x 65 x 8192, 3, 96 and 82; the line at 8 or 16 changes nothing more).
     // Where every CTA has one unit at most the weights would only move units together: 80 x 512 x 1024
     // 13.0 us without them, 13.6 with.
     p.strips_last = 2;
@@ -252,7 +255,7 @@ inline Cut make_cut(int m, int n, int k, int ksplit, int kb_split, CutMode mode,
         const int w = strips == 1 ? COST_1 : COST_2;
         const long long row = (long long)p.tiles_n * p.kblocks;
         const bool weigh = p.bands == 1 ? false
-                           : streamk    ? row * ((p.bands - 1ll) * COST + w) >= (long long)*grid * COST
+                           : streamk    ? row * ((p.bands - 1ll) * COST + w) >= 4ll * *grid * COST
                                         : units > sms;
         if (weigh) {
             p.w_full = COST;

@@ -173,6 +173,8 @@ def check_pieces(cut, m, n, k, sms):
         by_tile.setdefault(tile, []).append((kb0, kb1, index, pieces))
         corner.add((tile, band, u0, units, strips))
     assert sorted(by_tile) == list(range(tiles)) and len(corner) == tiles
+    # a short last band is weighed only where shares hold four whole units
+    assert c["w_last"] == c["w_full"] == 1 or c["length"] >= 4 * c["w_full"] * c["grid"]
     cover = np.zeros((c["bands"], c["ucols"]), np.int32)
     for (_, band, u0, units, strips) in corner:
         cover[band, u0:u0 + units] += 1
