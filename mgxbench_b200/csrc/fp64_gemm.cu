@@ -81,7 +81,7 @@ struct Params : Cut {
 };
 
 // Stream-K tickets: (launch tag << 8) | arrivals.  A ticket written by an earlier launch (another
-// tag), or never written, counts as no arrivals, so the tickets need no reset between launches.
+// tag), or never written, counts as no arrivals, so nothing clears the tickets before a launch.
 // Arrivals per tile are at most the grid size, below 256.
 __device__ __forceinline__ int ticket_count(unsigned long long *tk, unsigned long long tag)
 {
@@ -89,18 +89,18 @@ __device__ __forceinline__ int ticket_count(unsigned long long *tk, unsigned lon
     return (v >> 8) == tag ? (int)(v & 255u) : 0;
 }
 
-// Takes a ticket; returns the arrivals before this one, or -1 (status set) if the compare-and-swap
-// never got through (each failure is another arrival's success, so this does not happen).
+// Takes a ticket; returns the arrivals before this one.  The first to arrive replaces what an earlier launch left
+// by this launch's tag and no arrivals; only this launch's warps write here now, so whoever loses that
+// exchange finds the tag set, and each arrival is one addition.  (As one compare-and-swap per arrival,
+// all but one of the CTAs that arrive together failed each time and tried again: 128 x 128 x 4096, 74
+// pieces a tile, 81 us, 43 now.)
 __device__ __forceinline__ int ticket_take(unsigned long long *tk, unsigned long long tag, int *status)
 {
-    unsigned long long old = atomicAdd(tk, 0ull);
-    for (int it = 0; it < 4096; ++it) {
-        const unsigned long long cur = (old >> 8) == tag ? old : (tag << 8);
-        const unsigned long long prev = atomicCAS(tk, old, cur + 1);
-        if (prev == old) return (int)(cur & 255u);
-        old = prev;
-    }
-    record_status(status, kDevTicket);
+    const unsigned long long old = atomicAdd(tk, 0ull);
+    if ((old >> 8) != tag) atomicCAS(tk, old, tag << 8);
+    const unsigned long long prev = atomicAdd(tk, 1ull);
+    if ((prev >> 8) == tag) return (int)(prev & 255u);
+    record_status(status, kDevTicket);  // another launch uses the workspace at the same time
     return -1;
 }
 
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     // Bound by the trips to L2, one after the other because the pieces add up in order: 32
                     // loads are in flight at a time, two units of four pieces.  One by one, behind a test for the
                     // own piece (which has been written too, unless it is the first and never left its
-                    // registers), 128 x 128 x 4096 with 74 pieces took 335 us, 83 now, 256^3 with 8 35 and 15.
+                    // registers), 128 x 128 x 4096 with 74 pieces took 335 us against 82, 256^3 with 8 35 against 15.
                     constexpr int TRIP = 4;
 #pragma unroll
                     for (int i0 = 0; i0 < NACC; i0 += 8) {

@@ -29,3 +29,11 @@ def test_uncut_tiles_cost_no_more_than_whole_k(mgx):
     """One K block, no tile cut: 0.93 times the whole-K kernel's time; 1.6 when every item asked for its piece."""
     sk, whole = times(mgx, 1102, 19749, 3, (0, 1))
     assert sk < 1.3 * whole, (sk, whole)
+
+
+@pytest.mark.parametrize("m,n,k", [(128, 128, 4096), (64, 64, 65536), (300, 300, 300)])
+def test_many_pieces_do_not_cost_more_than_slices(mgx, m, n, k):
+    """Against eight K slices, whose sums are a kernel of their own.  With loads one by one and arrivals by
+    compare-and-swap the shapes took 19, 5 and 3.6 times as long as with slices."""
+    sk, slices = times(mgx, m, n, k, (0, 8))
+    assert sk < 2.5 * slices + 15, (sk, slices)
