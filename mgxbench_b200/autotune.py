@@ -29,8 +29,8 @@ from pathlib import Path
 
 import numpy as np
 
-# The FP64 kernel cuts every product in equal shares per SM: the tile heights of 128 and 64 rows that
-# ids 0, 2-5 and 9-12 name (of the kernel that the packaged sweep measured) now run alike.
+# The FP64 kernel cuts every product in equal shares per SM, so the tile heights of 128 and 64 rows run
+# alike: ids 9-12 are ids 0 and 2-4 by another name, and the models see them as those (SAME_KERNEL).
 TILE_FP64 = 0          # native FP64 kernel (DMMA), 128 rows, over the whole K range
 TILE_OZAKI_128 = 1     # Ozaki INT8 kernel, 128 x 128 output tiles over the whole K range
 # native FP64 kernel, 128 rows, K cut into 2 / 4 / 8 / 16 slices (split-K)
@@ -51,6 +51,9 @@ FP64_KSPLIT = {TILE_FP64: 1, TILE_FP64_K2: 2, TILE_FP64_K4: 4, TILE_FP64_K8: 8, 
 FP64_TILE_M = {TILE_FP64_T64: 64, TILE_FP64_T64_K2: 64, TILE_FP64_T64_K4: 64, TILE_FP64_T64_K8: 64,
                TILE_FP64_T64_SK: 64}
 OZAKI_KSPLIT = {TILE_OZAKI_128: 1, TILE_OZAKI_K4: 4, TILE_OZAKI_K16: 16}
+# ids that run the kernel of another (the same in host/autotune.h, model_tile)
+SAME_KERNEL = {TILE_FP64_T64: TILE_FP64, TILE_FP64_T64_K2: TILE_FP64_K2, TILE_FP64_T64_K4: TILE_FP64_K4,
+               TILE_FP64_T64_K8: TILE_FP64_K8}
 SPLITS = tuple(range(3, 10))
 CRT_MODULI = (9, 11, 12, 13, 14, 15, 16)
 CRT_KMAX = 130816
@@ -132,7 +135,8 @@ def candidates(m=None, n=None, k=None):
 
 
 def features(m, n, k, exp_range, cand: Candidate):
-    return [math.log2(m), math.log2(n), math.log2(k), float(exp_range), float(cand.tile), float(cand.splits)]
+    return [math.log2(m), math.log2(n), math.log2(k), float(exp_range),
+            float(SAME_KERNEL.get(cand.tile, cand.tile)), float(cand.splits)]
 
 
 # ------------------------------------------------------------------ measurements
@@ -243,7 +247,7 @@ class RegressionModel:
         self.rt = {}
         by = {}
         for r in rows:
-            by.setdefault((r["tile"], r["splits"]), []).append(r)
+            by.setdefault((SAME_KERNEL.get(r["tile"], r["tile"]), r["splits"]), []).append(r)
         for key, rs in by.items():
             x = np.array([math.log(r["m"] * r["n"] * r["k"]) for r in rs])
             y = np.array([math.log(r["seconds"]) for r in rs])
@@ -267,7 +271,7 @@ class RegressionModel:
     def predict(self, m, n, k, exp_range, cands):
         out = []
         for c in cands:
-            a, b = self.rt.get((c.tile, c.splits), (0.0, 1.0))
+            a, b = self.rt.get((SAME_KERNEL.get(c.tile, c.tile), c.splits), (0.0, 1.0))
             t = math.exp(a + b * math.log(m * n * k))
             e = self.err.get((c.form, c.splits, self._bucket(exp_range)))
             if e is None:

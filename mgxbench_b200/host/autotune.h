@@ -103,6 +103,19 @@ inline int tile_ksplit(int tile)
     }
 }
 
+// The id under which the model knows a candidate: 9-12 run the kernels of 0 and 2-4
+// (mgxbench_b200.autotune.SAME_KERNEL).
+inline int model_tile(int tile)
+{
+    switch (tile) {
+    case 9: return 0;
+    case 10: return 2;
+    case 11: return 3;
+    case 12: return 4;
+    default: return tile;
+    }
+}
+
 inline int tile_rows(int tile) { return (tile >= 9 && tile <= 13) ? 64 : 128; }
 inline bool tile_is_crt(int tile) { return tile == 8; }
 inline bool tile_is_fp64(int tile) { return tile != 1 && tile != 6 && tile != 7 && !tile_is_crt(tile); }
@@ -177,7 +190,7 @@ inline int auto_choose(const std::string &path, int m, int n, int k, double exp_
     std::vector<float> X((size_t)nc * 6), P(params.begin(), params.end()), Y((size_t)nc * 2);
     for (int c = 0; c < nc; ++c) {
         const double feat[6] = {std::log2((double)m), std::log2((double)n), std::log2((double)k), exp_range,
-                                cand[2 * c], cand[2 * c + 1]};
+                                (double)model_tile((int)cand[2 * c]), cand[2 * c + 1]};
         for (int j = 0; j < 6; ++j) X[(size_t)c * 6 + j] = (float)((feat[j] - xmean[j]) / xstd[j]);
     }
     float *dX = nullptr, *dP = nullptr, *dY = nullptr;
