@@ -30,3 +30,19 @@ def test_cpp_chooser_maps_the_same_ids():
     got = re.findall(r"case (\d+): return (\d+);", body[:body.index("}\n}")])
     assert sorted((int(b), int(a)) for a, b in got) == PAIRS
     assert re.search(r"feat\[6\] = \{[^}]*model_tile\(\(int\)cand\[2 \* c\]\)", text)
+
+
+def test_packaged_sweep_is_of_these_kernels():
+    """Both names of a kernel were measured alike, and the packaged network was trained on the packaged sweep."""
+    import json
+    import statistics
+    db = at.SweepDB(ROOT / "mgxbench_b200" / "data" / "sweep_b200.jsonl")
+    held = {}
+    for r in db.rows:
+        if r.get("set") == "heldout":
+            held.setdefault((r["m"], r["n"], r["k"], r["exp_range"]), {})[(r["tile"], r["splits"])] = r["seconds"]
+    for a, b in PAIRS:
+        ratios = [abs(math.log(d[a, 0] / d[b, 0])) for d in held.values() if (a, 0) in d and (b, 0) in d]
+        assert len(ratios) > 300 and statistics.median(ratios) < 0.05
+    model = json.loads((ROOT / "mgxbench_b200" / "data" / "mlp_b200.json").read_text())
+    assert model["training_set"] == db.digest()
