@@ -43,6 +43,6 @@ def test_packaged_sweep_is_of_these_kernels():
             held.setdefault((r["m"], r["n"], r["k"], r["exp_range"]), {})[(r["tile"], r["splits"])] = r["seconds"]
     for a, b in PAIRS:
         ratios = [abs(math.log(d[a, 0] / d[b, 0])) for d in held.values() if (a, 0) in d and (b, 0) in d]
-        assert len(ratios) > 300 and statistics.median(ratios) < 0.05
+        assert len(ratios) > 300 and statistics.quantiles(ratios, n=10)[-1] < 0.1
     model = json.loads((ROOT / "mgxbench_b200" / "data" / "mlp_b200.json").read_text())
     assert model["training_set"] == db.digest()
