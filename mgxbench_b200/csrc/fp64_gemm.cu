@@ -9,10 +9,10 @@
 //     band and all of the tile's columns, so a tile of any width up to 128 columns loads the four
 //     pipes equally and its time is proportional to its width (a last band of up to 32 rows is
 //     spread over them by columns, see COST).  The CTAs' shares of a product can then
-//     be equal to within one unit (Walk), whatever the shape.  Against whole 128 x 128 tiles dealt
-//     to the SMs: N = 256 (4 tiles on 148 SMs) 39 -> 7.5 us, N = 1024 (64 tiles) 145 -> 67 us,
-//     1024 x 4096 x 2048 (256 tiles: 1.73 waves paid as 2) 614 -> 493 us, N = 8192 35.1 -> 36.6
-//     TFLOP/s.
+//     be equal to within one unit (Walk), whatever the shape; fp64_cut.h has the cut.  Against whole
+//     128 x 128 tiles dealt to the SMs: N = 256 (4 tiles on 148 SMs) 39 -> 7.6 us a call, N = 1024 (64
+//     tiles) 145 -> 68 us, 1024 x 4096 x 2048 (256 tiles: 1.73 waves paid as 2) 614 -> 483 us, N = 8192
+//     35.1 -> 36.6 TFLOP/s.
 //   * warpgroup 0 (producer, one lane): TMA 2D loads of A (BM x 32 doubles) and B (32 x up to 128)
 //     into a ring of 128-byte swizzled tiles, each stage guarded by a full/empty mbarrier pair.  No
 //     multicast.  Operands TMA cannot describe (odd leading dimension or K offset, unaligned

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(THREADS) forward_kernel(const float *__restric
 
 // The same for large batches: one thread per sample, the parameters broadcast from shared memory.  A sample
 // group's two barriers and unit tiles cost more here than the tiles save: 131072 samples 61.2 us by
-// groups, 58.7 so; 1,000,000 446 and 365.  Smaller batches do not fill the SMs: 98304 46.2 and 49.3, 4096 4.5
+// groups, 56.7 so; 1,000,000 446 and 362.  Smaller batches do not fill the SMs: 98304 46.2 and 49.3, 4096 4.5
 // and 22.6.  Both add in the same order, so the rule changes no bit.
 constexpr int SAMPLE_THREADS_BATCH = 131072;
 

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(256) ozaki_zero(const ColStats z)
 // T threads per row, R rows per block (R > 1: a warp each), eight loads in flight per thread.  With one
 // warp per row for every k, a short, wide A occupied a few SMs: the split phase of 128 x 2000 x 16384 took
 // 318 us, 149 now.  With one row per block for every m, the blocks' starts took the time of a tall,
-// narrow A: 300000 x 64 x 64, 3 slices, 537 us, against 309 with eight.
+// narrow A: 300000 x 64 x 64, 3 slices, 537 us in all, 285 with eight.
 template <int T, int R>
 __global__ void __launch_bounds__(T * R) ozaki_row_exp(const double *__restrict__ A, int m, int k, int lda,
                                                        int *__restrict__ ea, const ColStats z, int *status)

@@ -260,8 +260,8 @@ __global__ void __launch_bounds__(T) crt_row_scale(const double *__restrict__ A,
 // It reads B before it waits for the kernel before it, the residues of A or the clearing of colmax: that
 // kernel writes nothing of B, and this one only starts once all its blocks have seen their own
 // predecessors complete.  So the scan fills the end of the residue pass: whole products at 1024^3 62.3
-// -> 58.3 us, 512^3 34.4 -> 31.8, 2501 x 1999 x 3001 317 -> 313.  The residue passes loading their
-// values before the wait gained nothing more (2501 x 1999 x 3001 321.8 against 319.9).
+// -> 58.3 us, 512^3 34.4 -> 31.8, 1.3% at 2501 x 1999 x 3001 (323 us in all).  The residue passes loading
+// their values before the wait gained nothing more.
 __global__ void __launch_bounds__(256) crt_col_max(const double *__restrict__ B, int k, int n, int ldb,
                                                    unsigned long long *colmax)
 {
