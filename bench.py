@@ -42,8 +42,8 @@ CHECK_ROWS = 256
 # captures (dram__bytes_read.sum + dram__bytes_write.sum) of bench.py at full size:
 # ozaki_gemm with s = 8 reads 83.69 GB and writes 2.15 GB; crt_gemm with q = 15 reads
 # 48.49 GB and writes 4.03 GB.  (At N = 8192 crt_gemm moves 5.67 GB, 1.88x its algorithmic bytes;
-# scaled by the algorithmic bytes that would be 22.7 GB at N = 16384, an underestimate because a modulus's operands outgrow L2, so the measured
-# full-size figure is kept.)
+# scaled by the algorithmic bytes that would be 22.7 GB at N = 16384, an underestimate because a
+# modulus's operands outgrow L2, so the measured full-size figure is kept.)
 OZAKI_GEMM_TRAFFIC_BYTES = 85.84e9
 CRT_GEMM_TRAFFIC_BYTES = 52.52e9
 
